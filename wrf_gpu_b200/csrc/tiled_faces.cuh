@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(TSX *TSY, WG_UFACE_MINB) k_uface_tiled(Grid g,
       return div_msf(ld(s.v, ix3(k, jv, ic, ny + 1, nx)) * (c1 * muv_c + c2), g.msfvx, g.rmsfvx, ix2(jv, ic, nx));
     };
     auto rwq = [&](int kf, int ic) {
-      return ld(s.w, ix3(kf, j, ic, ny, nx)) * (ld(g.c1f, kf) * mu2(j, ic) + ld(g.c2f, kf)) /
-             ld(g.msfty, ix2(j, ic, nx));
+      return div_msf(ld(s.w, ix3(kf, j, ic, ny, nx)) * (ld(g.c1f, kf) * mu2(j, ic) + ld(g.c2f, kf)), g.msfty,
+                     g.rmsfty, ix2(j, ic, nx));
     };
     const double f_u = 0.5 * (ld(g.f, ix2(j, l, nx)) + ld(g.f, ix2(j, r, nx)));
     const double e_u = 0.5 * (ld(g.e, ix2(j, l, nx)) + ld(g.e, ix2(j, r, nx)));
@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(TSX *TSY, WG_VFACE_MINB) k_vface_tiled(Grid g,
       return div_msf(ld(s.u, ix3(k, jc, iu, ny, nx + 1)) * (c1 * muu_c + c2), g.msfuy, g.rmsfuy, ix2(jc, iu, nx + 1));
     };
     auto rwq = [&](int kf, int jc) {
-      return ld(s.w, ix3(kf, jc, i, ny, nx)) * (ld(g.c1f, kf) * mu2(jc, i) + ld(g.c2f, kf)) /
-             ld(g.msfty, ix2(jc, i, nx));
+      return div_msf(ld(s.w, ix3(kf, jc, i, ny, nx)) * (ld(g.c1f, kf) * mu2(jc, i) + ld(g.c2f, kf)), g.msfty,
+                     g.rmsfty, ix2(jc, i, nx));
     };
     const double f_v = 0.5 * (ld(g.f, ix2(sj, i, nx)) + ld(g.f, ix2(nj, i, nx)));
     const double e_v = 0.5 * (ld(g.e, ix2(sj, i, nx)) + ld(g.e, ix2(nj, i, nx)));
