@@ -21,6 +21,11 @@ namespace wg {
 struct Acoustic {
   double *u, *v, *w, *ph, *theta_w, *t2ave, *p, *pm1, *al, *ww;  // evolving
   double *mu, *muts, *muave, *mudf;                              // evolving 2-D
+  // where the substep's results go: the arrays themselves (in place), or
+  // another set that receives every element (oop; advance_uv, k_div_h and the
+  // level-parallel column kernel)
+  double *u_o, *v_o, *w_o, *ph_o, *theta_o, *t2ave_o, *p_o, *pm1_o, *al_o, *ww_o, *mu_o, *muts_o, *muave_o, *mudf_o;
+  int oop;
   const double *u_tend, *v_tend, *t_tend, *rw_tend, *ph_tend;    // stage tendencies
   const double *alt, *pb, *c2a, *cqu, *cqv, *cqw, *php, *pt1;    // stage constants
   const double *a, *alpha, *gamma, *ww_1;
@@ -30,6 +35,12 @@ struct Acoustic {
   const double *theta_s;                                         // stage theta (t_save = theta - 300)
   const double *phb0;                                            // stage base geopotential at face 0 (ny, nx)
 };
+
+inline void in_place(Acoustic &A) {
+  A.u_o = A.u; A.v_o = A.v; A.w_o = A.w; A.ph_o = A.ph; A.theta_o = A.theta_w; A.t2ave_o = A.t2ave; A.p_o = A.p;
+  A.pm1_o = A.pm1; A.al_o = A.al; A.ww_o = A.ww; A.mu_o = A.mu; A.muts_o = A.muts; A.muave_o = A.muave;
+  A.mudf_o = A.mudf; A.oop = 0;
+}
 
 constexpr int BDY_MAX_ZONE = 16;
 
@@ -224,7 +235,7 @@ __global__ void __launch_bounds__(128, WG_UV_MINB) k_advance_uv(Grid g, Acoustic
         const double ms = c1 * ld(A.muus, fu) + c2, mc = c1 * ld(A.muu, fu) + c2;
         u = div_msf(strip_at(bdy.cad_u, nz, j == 0 ? 2 : 3, 0, k, i) * ms - ld(A.u_1, cu) * mc, g.msfuy, g.rmsfuy, fu);
       }
-      A.u[cu] = u;
+      A.u_o[cu] = u;
     }
     if (dv) {
       const int cv = k * vplane + fv;
@@ -246,7 +257,7 @@ __global__ void __launch_bounds__(128, WG_UV_MINB) k_advance_uv(Grid g, Acoustic
         const double ms = c1 * ld(A.muvs, fv) + c2, mc = c1 * ld(A.muv, fv) + c2;
         v = div_msf(strip_at(bdy.cad_v, nz, i == 0 ? 0 : 1, 0, k, j) * ms - ld(A.v_1, cv) * mc, g.msfvx, g.rmsfvx, fv);
       }
-      A.v[cv] = v;
+      A.v_o[cv] = v;
     }
     pCm = pC0; pWm = pW0; pSm = pS0;
     pC0 = pC1; pW0 = pW1; pS0 = pS1;
@@ -281,8 +292,8 @@ __global__ void WG_DIVH_BOUNDS k_div_h(Grid g, Acoustic A, int specified, double
   const size_t c2d = ix2(j, i, nx);
   const double msftx = ld(g.msftx, c2d), msfty = ld(g.msfty, c2d);
   const double c1 = ld(g.c1h, k), c2 = ld(g.c2h, k);
-  const double v_n = ld(A.v, ix3(k, j + 1, i, nyv, nx)), v_s = ld(A.v, ix3(k, j, i, nyv, nx));
-  const double u_e = ld(A.u, ix3(k, j, i + 1, ny, nxu)), u_w = ld(A.u, ix3(k, j, i, ny, nxu));
+  const double v_n = ld(A.v_o, ix3(k, j + 1, i, nyv, nx)), v_s = ld(A.v_o, ix3(k, j, i, nyv, nx));
+  const double u_e = ld(A.u_o, ix3(k, j, i + 1, ny, nxu)), u_w = ld(A.u_o, ix3(k, j, i, ny, nxu));
   const double vn = v_n + (c1 * ld(A.muv, ix2(j + 1, i, nx)) + c2) * ld(A.v_1, ix3(k, j + 1, i, nyv, nx)) *
                               ld(g.rmsfvx, ix2(j + 1, i, nx));
   const double vs = v_s + (c1 * ld(A.muv, ix2(j, i, nx)) + c2) * ld(A.v_1, ix3(k, j, i, nyv, nx)) *

@@ -512,6 +512,58 @@ int wrfgpu_step_launch_count(const wrfgpu_step_params *p, int *launches) {
 
 namespace {
 
+// The column kernel and its launch shape for a column width (params; 0: the
+// default, 1: one thread per column, 16 / 32: level lanes) and a level-lane
+// count (0: the default).
+struct ColumnLaunch {
+  void (*kernel)(Grid, Acoustic, ColArgs, const double *, const double *);
+  dim3 grid, block;
+  size_t smem;
+  bool too_tall;
+};
+
+template <int TX, bool PIN>
+void (*column_tiled_kernel(int np))(Grid, Acoustic, ColArgs, const double *, const double *) {
+  switch (np) {
+    case 1: case 2: return k_column_tiled<TX, 2, PIN>;
+    case 3: return k_column_tiled<TX, 3, PIN>;
+    case 4: return k_column_tiled<TX, 4, PIN>;
+    case 5: return k_column_tiled<TX, 5, PIN>;
+    case 6: return k_column_tiled<TX, 6, PIN>;
+    case 7: return k_column_tiled<TX, 7, PIN>;
+    default: return k_column_tiled<TX, 14, PIN>;
+  }
+}
+
+ColumnLaunch column_launch(int nx, int ny, int nz, int width, int lanes, bool pins) {
+  ColumnLaunch c{};
+  if (width == 1) {
+    c.kernel = pins ? k_column_stream<true> : k_column_stream<false>;
+    c.grid = dim3((nx + 31) / 32, (ny + CS_WARPS - 1) / CS_WARPS, 1);
+    c.block = dim3(32, CS_WARPS, 1);
+    c.smem = column_stream_smem_bytes(nz);
+    return c;
+  }
+  const int tx = width > 0 ? width : COL_DEFAULT_WIDTH;
+  c.too_tall = width != 16 && nz > COL_MAX_NZ;
+  int np = 0;
+  const int ty = column_tiled_lanes(nz, tx, lanes, np);
+  c.kernel = tx == 16 ? (pins ? column_tiled_kernel<16, true>(np) : column_tiled_kernel<16, false>(np))
+                      : (pins ? column_tiled_kernel<32, true>(np) : column_tiled_kernel<32, false>(np));
+  c.grid = dim3((nx + tx - 1) / tx, ny, 1);
+  c.block = dim3(tx, ty, 1);
+  c.smem = column_tiled_smem_bytes(nz, tx, np);
+  return c;
+}
+
+// Reserve the kernel's dynamic shared memory on the current device.
+int column_reserve(const ColumnLaunch &c) {
+  if (c.too_tall ||
+      cudaFuncSetAttribute(c.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem) != cudaSuccess)
+    return fail(WRFGPU_ERR_CUDA, "cannot reserve shared memory for the column kernel (nz too large)");
+  return WRFGPU_OK;
+}
+
 // The RK3 step.  The forecast lead is `lead_seconds` (host; NaN = no lead:
 // boundary forcing off), or with `lead_dev` set a device-resident lead read
 // by the kernels that interpolate boundary strips in time (`lead_seconds` is
@@ -578,9 +630,6 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
   const double dt = p.dt;
   const int ns = p.acoustic_substeps;
   const int kc = (p.march_levels == 5 || p.march_levels == 25) ? p.march_levels : MARCH_KC;
-  const int lanes = (p.column_lanes > 0) ? p.column_lanes : COL_TY;
-  const int cwidth = (p.column_width > 0) ? p.column_width : COL_DEFAULT_WIDTH;
-  const bool col_stream = cwidth == 1;  // one thread per column (column_stream.cuh)
   const double dt_rk[3] = {dt / 3.0, 0.5 * dt, dt};
   const double dts_rk[3] = {dt / 3.0, dt / (double)ns, dt / (double)ns};
   const int nsub[3] = {1, ns / 2 > 1 ? ns / 2 : 1, ns};
@@ -968,6 +1017,7 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
     A.mut = w.mut; A.muu = w.muu; A.muv = w.muv; A.muus = w.muus; A.muvs = w.muvs;
     A.mu_tend = (cad && stage == 0) ? w.mu_tend_s1 : base_mu;
     A.u_1 = s.u; A.v_1 = s.v; A.w_save = s.w; A.theta_s = s.theta; A.phb0 = w.phb0;
+    in_place(A);
     ColArgs ca{};
     ca.dts = dts; ca.epssm = p.epssm; ca.specified = specified ? 1 : 0; ca.top_lid = p.top_lid;
     ca.w_damping = p.w_damping; ca.damp_opt = p.damp_opt; ca.dampcoef = p.dampcoef; ca.zdamp = p.zdamp;
@@ -984,27 +1034,10 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
       ca.cad_ph = leaf_at_off(in->ph_bdy, cad ? dt_rk[stage] : 0.0);
       ca.ph_save = s.ph_pert;
     }
-    const size_t col_smem = col_stream ? column_stream_smem_bytes(nz) : column_tiled_smem_bytes(nz, cwidth);
     // the ring-0 pins are compiled into their own instantiations
-    const bool pins = cad || nest_ph_pin;
-#define WG_COL(TX, TY) (pins ? k_column_tiled<TX, TY, true> : k_column_tiled<TX, TY, false>)
-    auto kColumn = col_stream ? (pins ? k_column_stream<true> : k_column_stream<false>)
-                   : (cwidth == 16) ? ((lanes == 8)    ? WG_COL(16, 8)
-                                       : (lanes == 16) ? WG_COL(16, 16)
-                                       : (lanes == 17) ? WG_COL(16, 17)
-                                                       : WG_COL(16, 13))
-                                    : ((lanes == 8)    ? WG_COL(32, 8)
-                                       : (lanes == 16) ? WG_COL(32, 16)
-                                       : (lanes == 17) ? WG_COL(32, 17)
-                                                       : WG_COL(32, 13));
-#undef WG_COL
-    const dim3 col_grid = col_stream ? dim3((nx + 31) / 32, (ny + CS_WARPS - 1) / CS_WARPS, 1)
-                                     : dim3((nx + cwidth - 1) / cwidth, ny, 1);
-    const dim3 col_block = col_stream ? dim3(32, CS_WARPS, 1) : dim3(cwidth, lanes, 1);
+    const ColumnLaunch col = column_launch(nx, ny, nz, p.column_width, p.column_lanes, cad || nest_ph_pin);
     auto kAdvanceUV = cad ? k_advance_uv<true> : k_advance_uv<false>;
-    if (stage == 0 && cudaFuncSetAttribute(kColumn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)col_smem) !=
-                          cudaSuccess)
-      return fail(WRFGPU_ERR_CUDA, "cannot reserve shared memory for k_column_tiled (nz too large)");
+    if (stage == 0 && (rc = column_reserve(col)) != WRFGPU_OK) return rc;
     for (int it = 0; it < nsub[stage]; ++it) {
       PROF("k_advance_uv");
       kAdvanceUV<<<grd(nx + 1, ny + 1, (nz + UV_KC - 1) / UV_KC), blk2(), 0, stream>>>(g, A, dts, p.top_lid,
@@ -1014,7 +1047,7 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
       k_div_h<<<grd(nx, ny, nz), blk2(), 0, stream>>>(g, A, specified ? 1 : 0, w.dvdxi, w.hdiv);
       LAUNCH_CHECK("k_div_h");
       PROF("k_column");
-      kColumn<<<col_grid, col_block, col_smem, stream>>>(g, A, ca, w.dvdxi, w.hdiv);
+      col.kernel<<<col.grid, col.block, col.smem, stream>>>(g, A, ca, w.dvdxi, w.hdiv);
       LAUNCH_CHECK("k_column");
       if (cad) {
         PROF("k_spec_w");
@@ -1390,6 +1423,7 @@ Acoustic ac_state(const wrfgpu_acoustic_consts &c, double *const w[14]) {
   A.pt1 = c.pt1; A.a = c.a; A.alpha = c.alpha; A.gamma = c.gamma; A.ww_1 = c.ww_1;
   A.mut = c.mut; A.muu = c.muu; A.muv = c.muv; A.muus = c.muu; A.muvs = c.muv; A.mu_tend = c.mu_tend;
   A.u_1 = c.u_1; A.v_1 = c.v_1; A.w_save = c.w_save; A.theta_s = c.theta; A.phb0 = c.phb0;
+  in_place(A);
   return A;
 }
 
@@ -1409,10 +1443,14 @@ BdyArgs ac_bdy(const wrfgpu_step_params &p, const wrfgpu_acoustic_consts &c, dou
   return ba;
 }
 
-// Launch one forward substep over the work arrays w[14] (in place).
+// Launch one forward substep of the work arrays w[14] into o[14] (w itself:
+// in place; otherwise no array of o may be one of w).
 int ac_forward(const wrfgpu_step_params &p, const Grid &g, const wrfgpu_acoustic_consts &c, double *const w[14],
-               double dts, const AcLayout &L, cudaStream_t stream) {
+               double *const o[14], double dts, const AcLayout &L, cudaStream_t stream) {
   Acoustic A = ac_state(c, w);
+  A.u_o = o[0]; A.v_o = o[1]; A.w_o = o[2]; A.ph_o = o[3]; A.theta_o = o[4]; A.t2ave_o = o[5]; A.p_o = o[6];
+  A.pm1_o = o[7]; A.al_o = o[8]; A.ww_o = o[9]; A.mu_o = o[10]; A.muts_o = o[11]; A.muave_o = o[12]; A.mudf_o = o[13];
+  A.oop = o != w ? 1 : 0;
   const int specified = (p.run_boundary && !p.bc_ideal) ? 1 : 0;
   BdyArgs ba = ac_bdy(p, c, dts);
   ColArgs ca{};
@@ -1424,13 +1462,10 @@ int ac_forward(const wrfgpu_step_params &p, const Grid &g, const wrfgpu_acoustic
   if (int rc = check_launch("k_advance_uv")) return rc;
   k_div_h<<<grd(nx, ny, nz), blk2(), 0, stream>>>(g, A, specified, L.dvdxi, L.hdiv);
   if (int rc = check_launch("k_div_h")) return rc;
-  const size_t smem = column_tiled_smem_bytes(nz, COL_TX);
-  auto kColumn = k_column_tiled<COL_TX, COL_TY>;
-  if (cudaFuncSetAttribute(kColumn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-    return fail(WRFGPU_ERR_CUDA, "cannot reserve shared memory for k_column_tiled (nz too large)");
-  kColumn<<<dim3((nx + COL_TX - 1) / COL_TX, ny, 1), dim3(COL_TX, COL_TY, 1), smem, stream>>>(g, A, ca, L.dvdxi,
-                                                                                             L.hdiv);
-  return check_launch("k_column_tiled");
+  const ColumnLaunch col = column_launch(nx, ny, nz, 0, 0, false);
+  if (int rc = column_reserve(col)) return rc;
+  col.kernel<<<col.grid, col.block, col.smem, stream>>>(g, A, ca, L.dvdxi, L.hdiv);
+  return check_launch("k_column");
 }
 
 Grid ac_grid(const wrfgpu_step_params &p, const wrfgpu_metrics &m, const AcLayout &L) {
@@ -1470,7 +1505,7 @@ extern "C" int wrfgpu_acoustic_substep(const wrfgpu_step_params *p, const wrfgpu
   k_recip_msf<<<grd(p->nx + 1, p->ny + 1, 1), blk2(), 0, stream>>>(g, L.rmsf[0], L.rmsf[1], L.rmsf[2], L.rmsf[3],
                                                                  L.rmsf[4], L.rmsf[5]);
   if ((rc = check_launch("k_recip_msf"))) return rc;
-  if ((rc = ac_forward(*p, g, *c, w, dts, L, stream))) return rc;
+  if ((rc = ac_forward(*p, g, *c, w, w, dts, L, stream))) return rc;
   g_last_error.clear();
   return WRFGPU_OK;
 }
@@ -1510,12 +1545,8 @@ extern "C" int wrfgpu_acoustic_substep_vjp(const wrfgpu_step_params *p, const wr
     for (double *q : x1)
       if (q == nullptr) return fail(WRFGPU_ERR_NULL_POINTER, "an x_out pointer is NULL");
   } else {
-    for (int q = 0; q < 14; ++q) {
-      x1[q] = L.x1[q];
-      if (cudaMemcpyAsync(L.x1[q], xin[q], n[q] * sizeof(double), cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
-        return fail(WRFGPU_ERR_CUDA, "work state copy failed");
-    }
-    if ((rc = ac_forward(*p, g, *c, L.x1, dts, L, stream))) return rc;
+    for (int q = 0; q < 14; ++q) x1[q] = L.x1[q];
+    if ((rc = ac_forward(*p, g, *c, xin, x1, dts, L, stream))) return rc;
   }
   const int specified = (p->run_boundary && !p->bc_ideal) ? 1 : 0;
   if (specified && x_out != nullptr) {  // the forward dvdxi (the drain limiter's input) from the stored output

@@ -105,6 +105,36 @@ __device__ __forceinline__ double div_rcp(double a, double b, double rb) {
 __device__ __forceinline__ double div_msf(double a, const double *msf, const double *rmsf, size_t idx) {
   return div_rcp(a, __ldg(msf + idx), __ldg(rmsf + idx));
 }
+// q[n] = a[n] / b[n] for N independent quotients.  The `/` operator ends every
+// quotient in a branch to its special-case path, and the scheduler cannot
+// overlap work across it, so a thread's divisions run one latency after
+// another.  Here each quotient is: the hardware's approximate reciprocal y0
+// (PTX rcp.approx.ftz.f64), one third-order Newton step y = y0 + y0 (e + e^2),
+// e = 1 - b y0, and Markstein's correction of a*y as in div_rcp -- straight-line
+// code that overlaps across n.  One test covers the batch: operands outside
+// 2^-500 < |b| < 2^500, |a| < 2^500 (zeros of b, infinities and NaN among them)
+// send all N through `/`.  Inside that range the quotient is `/`'s bit for bit
+// (checked on the GPU against it), except that a zero a may give +0 for -0.
+__device__ __forceinline__ double div_fast(double a, double b, bool &special) {
+  const unsigned eb = (unsigned)__double2hiint(b) & 0x7ff00000u, ea = (unsigned)__double2hiint(a) & 0x7ff00000u;
+  special = special || eb - 0x20b00000u >= 0x3e800000u || ea >= 0x5f300000u;
+  double y0;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
+  const double e = __fma_rn(-b, y0, 1.0);
+  const double y = __fma_rn(y0, __fma_rn(e, e, e), y0);
+  const double q = __dmul_rn(a, y);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+template <int N>
+__device__ __forceinline__ void div_batch(const double (&a)[N], const double (&b)[N], double (&q)[N]) {
+  bool special = false;
+#pragma unroll
+  for (int n = 0; n < N; ++n) q[n] = div_fast(a[n], b[n], special);
+  if (special) {
+#pragma unroll
+    for (int n = 0; n < N; ++n) q[n] = a[n] / b[n];
+  }
+}
 constexpr double R60 = 1.0 / 60.0;
 constexpr double R12 = 1.0 / 12.0;
 constexpr double RG = 1.0 / G;

@@ -14,6 +14,19 @@ __global__ void k_div_check(const double *a, const double *b, const double *rb, 
   q_div[i] = a[i] / b[i];
 }
 
+// Groups of three neighbouring quotients as one div_batch.
+__global__ void k_div_batch_check(const double *a, const double *b, double *q_batch, double *q_div, long groups) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= groups) return;
+  const double n[3] = {a[3 * i], a[3 * i + 1], a[3 * i + 2]}, d[3] = {b[3 * i], b[3 * i + 1], b[3 * i + 2]};
+  double q[3];
+  wg::div_batch(n, d, q);
+  for (int t = 0; t < 3; ++t) {
+    q_batch[3 * i + t] = q[t];
+    q_div[3 * i + t] = n[t] / d[t];
+  }
+}
+
 }  // namespace
 
 // q_rcp[i] = div_rcp(a[i], b[i], rb[i]) and q_div[i] = a[i] / b[i] (CUDA's
@@ -24,5 +37,15 @@ extern "C" int wrfgpu_selftest_div_rcp(const double *a, const double *b, const d
   const int threads = 256;
   const long blocks = (n + threads - 1) / threads;
   k_div_check<<<(unsigned)blocks, threads, 0, stream>>>(a, b, rb, q_rcp, q_div, n);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+// q_batch = div_batch over groups of three and q_div = a / b, on device arrays
+// of 3 * groups doubles.
+extern "C" int wrfgpu_selftest_div_batch(const double *a, const double *b, double *q_batch, double *q_div,
+                                         long groups, cudaStream_t stream) {
+  if (groups <= 0) return 0;
+  const int threads = 256;
+  k_div_batch_check<<<(unsigned)((groups + threads - 1) / threads), threads, 0, stream>>>(a, b, q_batch, q_div, groups);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
