@@ -95,37 +95,57 @@ __device__ __forceinline__ double relax_weight_v(int j, int i, int y_len, int x_
 
 // ---------------------------------------------------------------------------
 // advance_uv (core/acoustic.py:626-786) on both face kinds of one horizontal
-// position (i, j), marching up a chunk of UV_KC levels: the u face at i
+// position (i, j), marching up a chunk of kc levels: the u face at i
 // (j < ny; acoustic.py:626-735) and the v face at j (i < nx; :737-750).
 // Both faces read the mass points C = (jc, ic), W = (jc, i-1) and
 // S = (j-1, ic), edge-clamped like the reference's face pairs (u uses W|C,
 // v uses S|C).  p and ph of the three points are carried up the chunk in
 // registers and the level-invariant 2-D terms are formed once, so a level
 // loads only its new plane values; every expression keeps the reference's
-// operation order.  Index space (nx+1) x (ny+1) x ceil(nz / UV_KC).
+// operation order.  Index space (nx+1) x (ny+1) x ceil(nz / kc).
 // ---------------------------------------------------------------------------
-// levels per thread: timed at 433 x 433 x 50 (bench CUDA events, ms/step):
-// 17 (three chunks of 50 levels) 2.80, 13 2.88, 10 2.91, 9 2.95, 25 2.94,
-// 50 3.00; 17 with 3 blocks per SM 3.30
-#ifndef WG_UV_KC
-#define WG_UV_KC 17
-#endif
-constexpr int UV_KC = WG_UV_KC;
 // resident 128-thread blocks per SM requested from the register allocator
 // (4: 128 registers; timed at 433 x 433 x 50 against 1 (164 registers) and 5)
 #ifndef WG_UV_MINB
 #define WG_UV_MINB 4
 #endif
 
+// Levels per thread.  A chunk costs its levels plus about one (the register
+// window and the 2-D terms), so a grid that fills the GPU many times over takes
+// the longest chunks; a small one is bound by the chunk's latency and takes the
+// shortest that still fit in one wave, or the number of waves that costs least.
+// Timed (us per launch, 433 x 433 x 50: 17 levels 280, 13 288, 10 291, 9 295,
+// 5 326, 3 359, 25 294, 50 300); against 17 levels for every grid:
+// 40 x 32 x 50 27.7 -> 10.7, 64 x 64 x 40 28.0 -> 14.4, 217 x 185 x 35
+// 70 -> 52, 150 x 150 x 45 47 -> 43.5 (256 x 256 x 50 and up unchanged).
+constexpr int UV_KC_MAX = 17;
+inline int advance_uv_levels(int nx, int ny, int nz) {
+  const double resident = 148.0 * WG_UV_MINB;  // blocks the GPU holds at once
+  const double tiles = (double)((nx + 1 + 31) / 32) * ((ny + 1 + 3) / 4);
+  int best = UV_KC_MAX;
+  double best_cost = 1.0e300;
+  for (int n = (nz + UV_KC_MAX - 1) / UV_KC_MAX; n <= nz; ++n) {
+    const int kc = (nz + n - 1) / n;
+    const double waves = tiles * ((nz + kc - 1) / kc) / resident;
+    const double cost = (waves < 4.0 ? ceil(waves) : waves) * (kc + 1.1);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = kc;
+    }
+  }
+  return best;
+}
+
 // PIN: compile in the boundary cadence's ring-0 tangential wind pins.
 template <bool PIN = false>
-__global__ void __launch_bounds__(128, WG_UV_MINB) k_advance_uv(Grid g, Acoustic A, double dts, int top_lid, BdyArgs bdy) {
+__global__ void __launch_bounds__(128, WG_UV_MINB) k_advance_uv(Grid g, Acoustic A, double dts, int top_lid, BdyArgs bdy,
+                                                                 int kc) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int nx = g.nx, ny = g.ny, nz = g.nz, nxu = nx + 1, nyv = ny + 1;
   if (i > nx || j > ny) return;
-  const int k0 = blockIdx.z * UV_KC;
-  const int k1 = min(k0 + UV_KC, nz);
+  const int k0 = blockIdx.z * kc;
+  const int k1 = min(k0 + kc, nz);
   const bool du = j < ny, dv = i < nx;
   const int ic = min(i, nx - 1), jc = min(j, ny - 1);
   const int oC = jc * nx + ic, oW = jc * nx + max(i - 1, 0), oS = max(j - 1, 0) * nx + ic;

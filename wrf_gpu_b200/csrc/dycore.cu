@@ -629,6 +629,7 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
   const bool specified = p.run_boundary && !p.bc_ideal;
   const double dt = p.dt;
   const int ns = p.acoustic_substeps;
+  const int uv_kc = advance_uv_levels(p.nx, p.ny, p.nz);
   const int kc = (p.march_levels == 5 || p.march_levels == 25) ? p.march_levels : MARCH_KC;
   const double dt_rk[3] = {dt / 3.0, 0.5 * dt, dt};
   const double dts_rk[3] = {dt / 3.0, dt / (double)ns, dt / (double)ns};
@@ -1040,8 +1041,8 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
     if (stage == 0 && (rc = column_reserve(col)) != WRFGPU_OK) return rc;
     for (int it = 0; it < nsub[stage]; ++it) {
       PROF("k_advance_uv");
-      kAdvanceUV<<<grd(nx + 1, ny + 1, (nz + UV_KC - 1) / UV_KC), blk2(), 0, stream>>>(g, A, dts, p.top_lid,
-                                                                                              ba);
+      kAdvanceUV<<<grd(nx + 1, ny + 1, (nz + uv_kc - 1) / uv_kc), blk2(), 0, stream>>>(g, A, dts, p.top_lid, ba,
+                                                                                       uv_kc);
       LAUNCH_CHECK("k_advance_uv");
       PROF("k_div_h");
       k_div_h<<<grd(nx, ny, nz), blk2(), 0, stream>>>(g, A, specified ? 1 : 0, w.dvdxi, w.hdiv);
@@ -1458,7 +1459,9 @@ int ac_forward(const wrfgpu_step_params &p, const Grid &g, const wrfgpu_acoustic
   ca.damp_opt = p.damp_opt; ca.dampcoef = p.dampcoef; ca.zdamp = p.zdamp;
   ca.rzdamp = (p.zdamp != 0.0 && std::isfinite(1.0 / p.zdamp)) ? 1.0 / p.zdamp : 0.0;
   const int nx = p.nx, ny = p.ny, nz = p.nz;
-  k_advance_uv<false><<<grd(nx + 1, ny + 1, (nz + UV_KC - 1) / UV_KC), blk2(), 0, stream>>>(g, A, dts, p.top_lid, ba);
+  const int uv_kc = advance_uv_levels(nx, ny, nz);
+  k_advance_uv<false><<<grd(nx + 1, ny + 1, (nz + uv_kc - 1) / uv_kc), blk2(), 0, stream>>>(g, A, dts, p.top_lid, ba,
+                                                                                          uv_kc);
   if (int rc = check_launch("k_advance_uv")) return rc;
   k_div_h<<<grd(nx, ny, nz), blk2(), 0, stream>>>(g, A, specified, L.dvdxi, L.hdiv);
   if (int rc = check_launch("k_div_h")) return rc;
