@@ -772,19 +772,20 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
     k_transport_tiled<<<dim3((nx + 31) / 32, ny, 1), dim3(32, 8, 1), transport_smem_bytes(nz), stream>>>(
         g, s.u, s.v, s.mu_total, w.ru, w.rv, w.rom, specified ? w.ww_spec : nullptr);
     LAUNCH_CHECK("k_transport");
-    Diag dg{w.alt_raw, w.alt, w.pb, w.c2a, w.qtot, w.al_ls, w.php_ls, w.php};
+    // (rw: in the acoustic ww array, which the w-face kernel fills afterwards)
+    Diag dg{w.alt_raw, w.alt, w.pb, w.c2a, w.qtot, w.al_ls, w.php_ls, w.php, w.ww};
     PROF("k_diag");
     k_diag<<<grd(nx, ny, nz), blk2(), 0, stream>>>(g, s, p.hypsometric_opt, dg);
     LAUNCH_CHECK("k_diag");
     UFaceOut uo{w.u_tend, w.u_w, w.cqu};
     PROF("k_uface");
     kUface<<<tgrd(nx + 1, ny, nz), tblk(), 0, stream>>>(g, s, origin, w.ru, w.rv, w.rom, dg, w.muu, w.muus,
-                                                               in->base_u, p.top_lid, p.run_boundary, uo);
+                                                               in->base_u, dg.rw, p.top_lid, p.run_boundary, uo);
     LAUNCH_CHECK("k_uface");
     VFaceOut vo{w.v_tend, w.v_w, w.cqv};
     PROF("k_vface");
     kVface<<<tgrd(nx, ny + 1, nz), tblk(), 0, stream>>>(g, s, origin, w.ru, w.rv, w.rom, dg, w.muv, w.muvs,
-                                                               in->base_v, p.top_lid, p.run_boundary, vo);
+                                                               in->base_v, dg.rw, p.top_lid, p.run_boundary, vo);
     LAUNCH_CHECK("k_vface");
     const bool lim_theta = (rk == 3) && (p.scalar_adv_opt == 1 || p.scalar_adv_opt == 2);
     const bool lim_moist = moist && (rk == 3) && (p.moist_adv_opt == 1 || p.moist_adv_opt == 2);

@@ -97,15 +97,20 @@ __global__ void k_mass2d(Grid g, StateR s, const double *ref_mu_pert, int rk_ste
 //   al_ls   = large-step al                  (rk_addtend_dry.py:186-224)
 //   php_ls  = 0.5*(pht(k)+pht(k+1))          (rk_addtend_dry.py:227-228)
 //   php     = stage-constant php             (small_step_prep.py:350-352)
+//   rw      = coupled w on the w faces       (rk_addtend_dry.py:405-466), formed
+//             once here for the Coriolis terms of the u and v faces (each cell's
+//             value enters eight of their quads: uface 2.30 -> 1.74, vface 2.17 ->
+//             1.62 ms/step at 433 x 433 x 50 together with the coupled u / v
+//             quads read from the staged tiles)
 // ---------------------------------------------------------------------------
 struct Diag {
-  double *alt_raw, *alt, *pb, *c2a, *qtot, *al_ls, *php_ls, *php;
+  double *alt_raw, *alt, *pb, *c2a, *qtot, *al_ls, *php_ls, *php, *rw;
 };
 
-// 16 resident blocks of 128 per SM (32 registers): timed at 433 x 433 x 50,
-// 0.696 vs 0.735 ms/step with the compiler's 56 registers (12: 0.721).
+// 12 resident blocks of 128 per SM (40 registers): timed at 433 x 433 x 50,
+// 0.79 vs 0.84 ms/step at 16 (32 registers, spills since rw was added).
 #ifndef WG_DIAG_MINB
-#define WG_DIAG_MINB 16
+#define WG_DIAG_MINB 12
 #endif
 #if WG_DIAG_MINB > 0
 #define WG_DIAG_BOUNDS __launch_bounds__(128, WG_DIAG_MINB)
@@ -122,6 +127,12 @@ __global__ void WG_DIAG_BOUNDS k_diag(Grid g, StateR s, int hyps, Diag o) {
   const size_t f0 = c, f1 = ix3(k + 1, j, i, ny, nx);
   const size_t c2d = ix2(j, i, nx);
   const double theta = ld(s.theta, c), pt = ld(s.p_total, c), pp = ld(s.p_pert, c);
+  const double mu_total = ld(s.mu_total, c2d), mu_pert = ld(s.mu_pert, c2d);
+  auto put_rw = [&](int f, size_t cf) {
+    o.rw[cf] = div_msf(ld(s.w, cf) * (ld(g.c1f, f) * mu_total + ld(g.c2f, f)), g.msfty, g.rmsfty, c2d);
+  };
+  put_rw(k, f0);
+  if (k == g.nz - 1) put_rw(k + 1, f1);
   const double alt_raw = inv_density(theta, pt);
   const double alt = dmax(alt_raw, MIN_ACOUSTIC_ALT);
   const double pb = pt - pp;
@@ -136,7 +147,6 @@ __global__ void WG_DIAG_BOUNDS k_diag(Grid g, StateR s, int hyps, Diag o) {
   o.qtot[c] = qt;
   const double ph0 = ld(s.ph_pert, f0), ph1 = ld(s.ph_pert, f1);
   const double phb0 = ld(s.ph_total, f0) - ph0, phb1 = ld(s.ph_total, f1) - ph1;
-  const double mu_total = ld(s.mu_total, c2d), mu_pert = ld(s.mu_pert, c2d);
   const double mub = mu_total - mu_pert;
   const double c1 = ld(g.c1h, k), c2 = ld(g.c2h, k), rdnw = ld(g.rdnw, k);
   double al;

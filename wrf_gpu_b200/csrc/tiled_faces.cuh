@@ -126,8 +126,8 @@ template <typename F, bool DEG>
 __global__ void __launch_bounds__(TSX *TSY, WG_UFACE_MINB) k_uface_tiled(Grid g, StateR s, StateR ref, const double *ru,
                                                            const double *rv, const double *rom, Diag d,
                                                            const double *muu, const double *muus,
-                                                           const double *base_u, int top_lid, int run_boundary,
-                                                           UFaceOut o) {
+                                                           const double *base_u, const double *rw, int top_lid,
+                                                           int run_boundary, UFaceOut o) {
   constexpr bool deg = DEG;  // the specified-boundary advection degradation
   using TQ = Tile<3, 3>;
   using TR = Tile<1, 0>;
@@ -239,17 +239,20 @@ __global__ void __launch_bounds__(TSX *TSY, WG_UFACE_MINB) k_uface_tiled(Grid g,
       const double muv_c = 0.5 * (mu2(js, ic) + mu2(jn, ic));
       return div_msf(ld(s.v, ix3(k, jv, ic, ny + 1, nx)) * (c1 * muv_c + c2), g.msfvx, g.rmsfvx, ix2(jv, ic, nx));
     };
-    auto rwq = [&](int kf, int ic) {
-      return div_msf(ld(s.w, ix3(kf, j, ic, ny, nx)) * (ld(g.c1f, kf) * mu2(j, ic) + ld(g.c2f, kf)), g.msfty,
-                     g.rmsfty, ix2(j, ic, nx));
-    };
+    auto rwq = [&](int kf, int ic) { return ld(rw, ix3(kf, j, ic, ny, nx)); };
     const double f_u = 0.5 * (ld(g.f, ix2(j, l, nx)) + ld(g.f, ix2(j, r, nx)));
     const double e_u = 0.5 * (ld(g.e, ix2(j, l, nx)) + ld(g.e, ix2(j, r, nx)));
     const double cosa_u = 0.5 * (ld(g.cosa, ix2(j, l, nx)) + ld(g.cosa, ix2(j, r, nx)));
     const double msf_u = div_msf(ld(g.msfux, ix2(j, i, nxu)), g.msfuy, g.rmsfuy, ix2(j, i, nxu));
     double ru_cor = 0.0;
     if (f_u != 0.0 || e_u != 0.0) {
-      const double rv_quad = 0.25 * (rvq(j, l) + rvq(j, r) + rvq(j + 1, l) + rvq(j + 1, r));
+      // away from the domain's edges the coupled v at the four points is the
+      // transport velocity of the staged tile (the same expression)
+      auto RVT = [&](int rr, int cc) { return srv[(rr + 1) * TV::W + (cc + 1)]; };
+      const bool in = i >= 1 && i <= nx - 1 && j >= 1 && j <= ny - 2;
+      const double rv_quad =
+          0.25 * (in ? RVT(ty, tx - 1) + RVT(ty, tx) + RVT(ty + 1, tx - 1) + RVT(ty + 1, tx)
+                     : rvq(j, l) + rvq(j, r) + rvq(j + 1, l) + rvq(j + 1, r));
       ru_cor = msf_u * f_u * rv_quad;
       const double rw_quad = 0.25 * (rwq(k, l) + rwq(k + 1, l) + rwq(k, r) + rwq(k + 1, r));
       ru_cor = ru_cor - e_u * cosa_u * rw_quad;
@@ -276,8 +279,8 @@ template <typename F, bool DEG>
 __global__ void __launch_bounds__(TSX *TSY, WG_VFACE_MINB) k_vface_tiled(Grid g, StateR s, StateR ref, const double *ru,
                                                            const double *rv, const double *rom, Diag d,
                                                            const double *muv, const double *muvs,
-                                                           const double *base_v, int top_lid, int run_boundary,
-                                                           VFaceOut o) {
+                                                           const double *base_v, const double *rw, int top_lid,
+                                                           int run_boundary, VFaceOut o) {
   constexpr bool deg = DEG;  // the specified-boundary advection degradation
   using TQ = Tile<3, 3>;
   using TR = Tile<1, 1>;
@@ -379,17 +382,18 @@ __global__ void __launch_bounds__(TSX *TSY, WG_VFACE_MINB) k_vface_tiled(Grid g,
       const double muu_c = 0.5 * (mu2(jc, il) + mu2(jc, ir));
       return div_msf(ld(s.u, ix3(k, jc, iu, ny, nx + 1)) * (c1 * muu_c + c2), g.msfuy, g.rmsfuy, ix2(jc, iu, nx + 1));
     };
-    auto rwq = [&](int kf, int jc) {
-      return div_msf(ld(s.w, ix3(kf, jc, i, ny, nx)) * (ld(g.c1f, kf) * mu2(jc, i) + ld(g.c2f, kf)), g.msfty,
-                     g.rmsfty, ix2(jc, i, nx));
-    };
+    auto rwq = [&](int kf, int jc) { return ld(rw, ix3(kf, jc, i, ny, nx)); };
     const double f_v = 0.5 * (ld(g.f, ix2(sj, i, nx)) + ld(g.f, ix2(nj, i, nx)));
     const double e_v = 0.5 * (ld(g.e, ix2(sj, i, nx)) + ld(g.e, ix2(nj, i, nx)));
     const double sina_v = 0.5 * (ld(g.sina, ix2(sj, i, nx)) + ld(g.sina, ix2(nj, i, nx)));
     const double msf_v = div_msf(ld(g.msfvy, ix2(j, i, nx)), g.msfvx, g.rmsfvx, ix2(j, i, nx));
     double rv_cor;
     if (f_v != 0.0 || e_v != 0.0) {
-      const double ru_quad = 0.25 * (ruq(sj, i) + ruq(sj, i + 1) + ruq(nj, i) + ruq(nj, i + 1));
+      // (as for the u faces: the coupled u is the staged transport velocity)
+      auto RUT = [&](int rr, int cc) { return sru[(rr + 1) * TR::W + (cc + 1)]; };
+      const bool in = i >= 1 && i <= nx - 2 && j >= 1 && j <= ny - 1;
+      const double ru_quad = 0.25 * (in ? RUT(ty - 1, tx) + RUT(ty - 1, tx + 1) + RUT(ty, tx) + RUT(ty, tx + 1)
+                                        : ruq(sj, i) + ruq(sj, i + 1) + ruq(nj, i) + ruq(nj, i + 1));
       rv_cor = -msf_v * f_v * ru_quad;
       const double rw_quad = 0.25 * (rwq(k, sj) + rwq(k + 1, sj) + rwq(k, nj) + rwq(k + 1, nj));
       rv_cor = rv_cor + msf_v * e_v * sina_v * rw_quad;

@@ -23,15 +23,29 @@ struct Tile {
 };
 
 // Stage one plane tile: element (r, c) holds src[wrap(j0-HY+r), wrap(i0-HX+c)] - sub.
+// A thread's elements are loaded together before the first is stored, and a
+// tile inside the domain skips the wraps (a compare chain per element).
 template <int HX, int HY>
 __device__ __forceinline__ void load_tile(double *t, const double *plane, int pitch, int i0, int j0, int px, int py,
                                           double sub) {
   using T = Tile<HX, HY>;
-  for (int e = threadIdx.y * TSX + threadIdx.x; e < T::N; e += TSX * TSY) {
-    const int r = e / T::W, c = e - r * T::W;
-    const int jj = wrp(j0 - HY + r, py), ii = wrp(i0 - HX + c, px);
-    t[e] = __ldg(plane + (size_t)jj * pitch + ii) - sub;
+  constexpr int NS = (T::N + TSX * TSY - 1) / (TSX * TSY);
+  const int tid = threadIdx.y * TSX + threadIdx.x;
+  const bool inside = i0 >= HX && j0 >= HY && i0 + TSX + HX <= px && j0 + TSY + HY <= py;
+  const int corner = (j0 - HY) * pitch + i0 - HX;
+  double v[NS];
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    const int e = tid + n * TSX * TSY;
+    if (e < T::N) {
+      const int r = e / T::W, c = e - r * T::W;
+      const int o = inside ? corner + r * pitch + c : wrp(j0 - HY + r, py) * pitch + wrp(i0 - HX + c, px);
+      v[n] = __ldg(plane + o);
+    }
   }
+#pragma unroll
+  for (int n = 0; n < NS; ++n)
+    if (tid + n * TSX * TSY < T::N) t[tid + n * TSX * TSY] = v[n] - sub;
 }
 
 // ---------------------------------------------------------------------------
