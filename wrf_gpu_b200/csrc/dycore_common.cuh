@@ -135,6 +135,13 @@ __device__ __forceinline__ void div_batch(const double (&a)[N], const double (&b
     for (int n = 0; n < N; ++n) q[n] = a[n] / b[n];
   }
 }
+// One such quotient (shorter than `/`; alone it does not overlap anything).
+__device__ __forceinline__ double div_one(double a, double b) {
+  const double n[1] = {a}, d[1] = {b};
+  double q[1];
+  div_batch(n, d, q);
+  return q[0];
+}
 constexpr double R60 = 1.0 / 60.0;
 constexpr double R12 = 1.0 / 12.0;
 constexpr double RG = 1.0 / G;
