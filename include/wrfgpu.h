@@ -400,6 +400,14 @@ int wrfgpu_acoustic_substep(const wrfgpu_step_params *params, const wrfgpu_metri
                             const wrfgpu_acoustic_consts *consts, wrfgpu_acoustic_work *x, double dts,
                             void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
+/* x_out <- one acoustic substep of x, which is left as it is (no array of
+ * x_out may be one of x); otherwise as wrfgpu_acoustic_substep.  For callers
+ * that keep the substep's input, who otherwise copy it first. */
+int wrfgpu_acoustic_substep_into(const wrfgpu_step_params *params, const wrfgpu_metrics *metrics,
+                                 const wrfgpu_acoustic_consts *consts, const wrfgpu_acoustic_work *x,
+                                 wrfgpu_acoustic_work *x_out, double dts, void *workspace, size_t workspace_bytes,
+                                 cudaStream_t stream);
+
 /* Cotangents of the stage tendencies the substep reads (wrfgpu_acoustic_consts
  * u_tend .. ph_tend, mu_tend), shaped like them; a NULL member is not
  * computed. */

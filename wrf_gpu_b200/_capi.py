@@ -141,7 +141,7 @@ EXPORTED = ("wrfgpu_step_params_init", "wrfgpu_step_params_validate", "wrfgpu_st
             "wrfgpu_rk3_step_batched", "wrfgpu_autotune", "wrfgpu_scalar_advection",
             "wrfgpu_scalar_advection_adjoint", "wrfgpu_scalar_advection_vjp", "wrfgpu_flux_advection",
             "wrfgpu_flux_advection_vjp", "wrfgpu_w_vertical_advection", "wrfgpu_w_vertical_advection_vjp",
-            "wrfgpu_acoustic_workspace_size", "wrfgpu_acoustic_substep",
+            "wrfgpu_acoustic_workspace_size", "wrfgpu_acoustic_substep", "wrfgpu_acoustic_substep_into",
             "wrfgpu_acoustic_substep_vjp", "wrfgpu_apply_lateral_boundaries",
             "wrfgpu_step_epilogue_workspace_size", "wrfgpu_step_epilogue", "wrfgpu_step_epilogue_device_lead", "wrfgpu_step_launch_count", "wrfgpu_profile_enable", "wrfgpu_profile_read",
             "wrfgpu_profile_class_count", "wrfgpu_profile_class_name", "wrfgpu_last_error_string",
@@ -212,6 +212,10 @@ def load(path: str | os.PathLike | None = None):
                                             ctypes.POINTER(AcousticConsts), ctypes.POINTER(AcousticWork), _D, _P,
                                             ctypes.c_size_t, _P]
     lib.wrfgpu_acoustic_substep.restype = _I
+    lib.wrfgpu_acoustic_substep_into.argtypes = [ctypes.POINTER(StepParams), ctypes.POINTER(Metrics),
+                                                 ctypes.POINTER(AcousticConsts), ctypes.POINTER(AcousticWork),
+                                                 ctypes.POINTER(AcousticWork), _D, _P, ctypes.c_size_t, _P]
+    lib.wrfgpu_acoustic_substep_into.restype = _I
     lib.wrfgpu_acoustic_substep_vjp.argtypes = [ctypes.POINTER(StepParams), ctypes.POINTER(Metrics),
                                                 ctypes.POINTER(AcousticConsts), ctypes.POINTER(AcousticWork),
                                                 ctypes.POINTER(AcousticWork), ctypes.POINTER(AcousticWork),

@@ -208,6 +208,17 @@ class AcousticOp:
             self.dts, ctypes.c_void_p(self.workspace.data_ptr()), self.workspace.numel(),
             ctypes.c_void_p(st.cuda_stream)))
 
+    def forward(self, xs) -> list:
+        """The 14 work tensors one substep on, in new tensors; ``xs`` is left as it is."""
+        out = [torch.empty_like(t) for t in xs]
+        x, o = self._work(xs), self._work(out)
+        st = torch.cuda.current_stream(xs[0].device)
+        _capi.check(self.lib.wrfgpu_acoustic_substep_into(
+            ctypes.byref(self.params), ctypes.byref(self.metrics), ctypes.byref(self.consts), ctypes.byref(x),
+            ctypes.byref(o), self.dts, ctypes.c_void_p(self.workspace.data_ptr()), self.workspace.numel(),
+            ctypes.c_void_p(st.cuda_stream)))
+        return out
+
     def vjp(self, xs, cot_out, x_out=None, tendencies=False):
         """Cotangents of the 14 inputs ``xs`` from those of the outputs;
         ``x_out`` (the substep's outputs from ``xs``) is recomputed if None.
@@ -233,8 +244,7 @@ class AcousticSubstep(torch.autograd.Function):
     @staticmethod
     def forward(ctx, op: AcousticOp, *xs):
         x_in = [t.contiguous() for t in xs]
-        out = [t.clone() for t in x_in]
-        op.forward_(out)
+        out = op.forward(x_in)
         ctx.op = op
         ctx.save_for_backward(*x_in, *out)
         return tuple(out)
@@ -256,8 +266,8 @@ class AcousticLoop(torch.autograd.Function):
     @staticmethod
     def forward(ctx, op: AcousticOp, nsub: int, *xs):
         x0 = [t.contiguous() for t in xs]
-        cur = [t.clone() for t in x0]
-        for _ in range(nsub):
+        cur = op.forward(x0) if nsub > 0 else [t.clone() for t in x0]
+        for _ in range(1, nsub):
             op.forward_(cur)
         ctx.op, ctx.nsub = op, nsub
         ctx.save_for_backward(*x0)
@@ -268,9 +278,7 @@ class AcousticLoop(torch.autograd.Function):
         x0 = list(ctx.saved_tensors)
         states = [x0]
         for _ in range(ctx.nsub):
-            nxt = [t.clone() for t in states[-1]]
-            ctx.op.forward_(nxt)
-            states.append(nxt)
+            states.append(ctx.op.forward(states[-1]))
         co = [g.contiguous() if g is not None else torch.zeros_like(x) for g, x in zip(grads, states[-1])]
         for n in range(ctx.nsub - 1, -1, -1):
             co = ctx.op.vjp(states[n], co, states[n + 1])

@@ -94,7 +94,7 @@ __global__ void WG_ADJCOL_BOUNDS k_adj_column(Grid g, AdjColArgs q) {
   const bool active = !q.specified || (j >= 1 && j <= ny - 2 && i >= 1 && i <= nx - 2);
   auto T1 = [&](int k) { return ld(q.theta_s, M(k)) - T0; };
   auto coef = [&](int k) {  // advance_w's stage-constant c2a*rdnw/mass_h(mut)
-    return ld(q.c2a, M(k)) * ld(g.rdnw, k) / safe12(ld(g.c1h, k) * mut + ld(g.c2h, k));
+    return div_one(ld(q.c2a, M(k)) * ld(g.rdnw, k), safe12(ld(g.c1h, k) * mut + ld(g.c2h, k)));
   };
   double *__restrict__ s_thw = q.s.gthw;
   double *__restrict__ s_rhs = q.s.grhs;
@@ -133,7 +133,10 @@ __global__ void WG_ADJCOL_BOUNDS k_adj_column(Grid g, AdjColArgs q) {
       const double den = safe * sttr;
       // the sweep is serial per column: one reciprocal per divisor instead
       // of six divisions on its dependency chain
-      const double rsafe = 1.0 / safe, rden = 1.0 / den;
+      const double one[2] = {1.0, 1.0}, dd[2] = {safe, den};
+      double rr[2];
+      div_batch(one, dd, rr);
+      const double rsafe = rr[0], rden = rr[1];
       const double thw = ld(q.x1.theta_w, c), al = ld(q.x1.al, c);
       const double g_mu_term = -(c2a * alt * t1 * rden) * g_pp - (alt * rsafe) * g_al;
       const double g_safe = -(c2a * alt * (thw - mu_term * t1) * (rsafe * rden)) * g_pp - (al * rsafe) * g_al;
@@ -149,7 +152,7 @@ __global__ void WG_ADJCOL_BOUNDS k_adj_column(Grid g, AdjColArgs q) {
       // ph finish: ph'(f) = rhs(f) + K ws(f) / (c1f muts + c2f)
       const double g_phn = ld(q.co.ph, c) - gal_prev + gal;
       const double mfs = ld(g.c1f, f) * muts + ld(g.c2f, f);
-      const double rmfs = 1.0 / mfs;
+      const double rmfs = div_one(1.0, mfs);
       s_rhs[c] = g_phn;
       double g_ws = ld(q.co.w, c) + (K * rmfs) * g_phn;
       g_muts += -(K * ld(q.x1.w, c) * ld(g.c1f, f) * (rmfs * rmfs)) * g_phn;
@@ -175,7 +178,7 @@ __global__ void WG_ADJCOL_BOUNDS k_adj_column(Grid g, AdjColArgs q) {
   auto predictor = [&](int f, double grhs, double &gph, double &gw, double &gwd_f, double &gwd_fm1) {
     if (f == nz && q.col.top_lid) grhs = 0.0;  // a rigid lid's rhs(nz) is zero
     gph += grhs;
-    const double S = msfty * grhs / (ld(g.c1f, f) * mut + ld(g.c2f, f));
+    const double S = div_one(msfty * grhs, ld(g.c1f, f) * mut + ld(g.c2f, f));
     gw += S * wfac;
     if (q.tc.ph_tend != nullptr) q.tc.ph_tend[M(f)] = dts * S;
     gwd_f = (f < nz) ? -(S * dts * ld(g.fnm, f)) : 0.0;
@@ -194,7 +197,7 @@ __global__ void WG_ADJCOL_BOUNDS k_adj_column(Grid g, AdjColArgs q) {
     const double c1 = ld(g.c1h, k);
     const double mass_h = c1 * muts + ld(g.c2h, k);
     const double t1 = T1(k);
-    const double rd = 1.0 / (mass_h * (T0 + t1));
+    const double rd = div_one(1.0, mass_h * (T0 + t1));
     const double gn = gt2a * rd;
     const double gthw = s_thw[c] + 0.5 * eps_p * gn;
     q.ci.t2ave[c] = 0.5 * eps_m * gn;

@@ -1501,16 +1501,20 @@ extern "C" int wrfgpu_acoustic_workspace_size(const wrfgpu_step_params *p, size_
   return WRFGPU_OK;
 }
 
-extern "C" int wrfgpu_acoustic_substep(const wrfgpu_step_params *p, const wrfgpu_metrics *m,
-                                       const wrfgpu_acoustic_consts *c, wrfgpu_acoustic_work *x, double dts,
-                                       void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+namespace {
+int ac_substep(const wrfgpu_step_params *p, const wrfgpu_metrics *m, const wrfgpu_acoustic_consts *c,
+               const wrfgpu_acoustic_work *x, const wrfgpu_acoustic_work *x_out, double dts, void *workspace,
+               size_t workspace_bytes, cudaStream_t stream) {
   int rc = ac_check(p, m, c, workspace_bytes, workspace);
   if (rc) return rc;
-  if (x == nullptr) return fail(WRFGPU_ERR_NULL_POINTER, "work state is NULL");
-  double *w[14];
+  if (x == nullptr || x_out == nullptr) return fail(WRFGPU_ERR_NULL_POINTER, "work state is NULL");
+  double *w[14], *o[14];
   work_ptrs(*x, w);
-  for (double *q : w)
-    if (q == nullptr) return fail(WRFGPU_ERR_NULL_POINTER, "a work state pointer is NULL");
+  work_ptrs(*x_out, o);
+  for (int q = 0; q < 14; ++q) {
+    if (w[q] == nullptr || o[q] == nullptr) return fail(WRFGPU_ERR_NULL_POINTER, "a work state pointer is NULL");
+    if (x != x_out && w[q] == o[q]) return fail(WRFGPU_ERR_BAD_SHAPE, "x_out must not alias x");
+  }
   Carver cv{reinterpret_cast<char *>(workspace), 0, workspace_bytes, false};
   AcLayout L;
   ac_carve(*p, cv, L);
@@ -1518,9 +1522,24 @@ extern "C" int wrfgpu_acoustic_substep(const wrfgpu_step_params *p, const wrfgpu
   k_recip_msf<<<grd(p->nx + 1, p->ny + 1, 1), blk2(), 0, stream>>>(g, L.rmsf[0], L.rmsf[1], L.rmsf[2], L.rmsf[3],
                                                                  L.rmsf[4], L.rmsf[5]);
   if ((rc = check_launch("k_recip_msf"))) return rc;
-  if ((rc = ac_forward(*p, g, *c, w, w, dts, L, stream))) return rc;
+  if ((rc = ac_forward(*p, g, *c, w, x == x_out ? w : o, dts, L, stream))) return rc;
   g_last_error.clear();
   return WRFGPU_OK;
+}
+}  // namespace
+
+extern "C" int wrfgpu_acoustic_substep(const wrfgpu_step_params *p, const wrfgpu_metrics *m,
+                                       const wrfgpu_acoustic_consts *c, wrfgpu_acoustic_work *x, double dts,
+                                       void *workspace, size_t workspace_bytes, cudaStream_t stream) {
+  return ac_substep(p, m, c, x, x, dts, workspace, workspace_bytes, stream);
+}
+
+extern "C" int wrfgpu_acoustic_substep_into(const wrfgpu_step_params *p, const wrfgpu_metrics *m,
+                                            const wrfgpu_acoustic_consts *c, const wrfgpu_acoustic_work *x,
+                                            wrfgpu_acoustic_work *x_out, double dts, void *workspace,
+                                            size_t workspace_bytes, cudaStream_t stream) {
+  if (x != nullptr && x == x_out) return fail(WRFGPU_ERR_BAD_SHAPE, "x_out must not alias x");
+  return ac_substep(p, m, c, x, x_out, dts, workspace, workspace_bytes, stream);
 }
 
 extern "C" int wrfgpu_acoustic_substep_vjp(const wrfgpu_step_params *p, const wrfgpu_metrics *m,
