@@ -562,11 +562,30 @@ __global__ void k_adj_uv_cols(Grid g, AdjUVArgs q) {
   if (i >= nx || j >= ny) return;
   const CellFaces cf(i, j, nx, ny);
   double muts = 0.0, mudf = 0.0;
-  for (int k = 0; k < nz; ++k) {
-    const double c1 = ld(g.c1h, k);
-    for (int n = 0; n < 4; ++n) {
-      muts = muts + cf.sw[n] * (-0.5 * c1 * cf.F(q, n, 1, k));
-      mudf = mudf + cf.dw[n] * cf.F(q, n, 2, k);
+  // KB levels' loads (8 each) issued before the first add: the sums are one
+  // chain, but their operands do not depend on it (256 x 256 x 50)
+  constexpr int KB = 4;
+  for (int k0 = 0; k0 < nz; k0 += KB) {
+    double f1[KB][4], f2[KB][4], c1[KB];
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      const int k = min(k0 + u, nz - 1);
+      c1[u] = ld(g.c1h, k);
+#pragma unroll
+      for (int n = 0; n < 4; ++n) {
+        f1[u][n] = cf.F(q, n, 1, k);
+        f2[u][n] = cf.F(q, n, 2, k);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      if (k0 + u < nz) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+          muts = muts + cf.sw[n] * (-0.5 * c1[u] * f1[u][n]);
+          mudf = mudf + cf.dw[n] * f2[u][n];
+        }
+      }
     }
   }
   const size_t c2d = (size_t)j * nx + i;
