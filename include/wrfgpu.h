@@ -80,7 +80,8 @@ typedef struct wrfgpu_step_params {
   double cf1, cf2, cf3, p_top;
   /* top-face extrapolation weights of the large-step PGF
    * (core/rk_addtend_dry.py:282-288): cfn = (0.5*dnw[nz-1] + dn[nz-1])/dn[nz-1],
-   * cfn1 = -0.5*dnw[nz-1]/dn[nz-1] */
+   * cfn1 = -0.5*dnw[nz-1]/dn[nz-1]; cfn = NaN: formed on the device from the
+   * metrics' dn and dnw */
   double cfn, cfn1;
   /* Kernel tile shapes (no counterpart in the reference; results do not
    * depend on them): levels per block of the level-marching stencil kernels

@@ -180,6 +180,7 @@ Grid make_grid(const wrfgpu_step_params &p, const wrfgpu_metrics &m, const doubl
   g.f = m.f; g.e = m.e; g.sina = m.sina; g.cosa = m.cosa;
   g.cf1 = p.cf1; g.cf2 = p.cf2; g.cf3 = p.cf3; g.p_top = p.p_top;
   g.cfn = p.cfn; g.cfn1 = p.cfn1;
+  g.cfn_from_dn = (std::isnan(p.cfn) && m.dn != nullptr && m.dnw != nullptr) ? 1 : 0;
   return g;
 }
 

@@ -43,7 +43,21 @@ struct Grid {
   const double *rmsftx, *rmsfty, *rmsfux, *rmsfuy, *rmsfvx, *rmsfvy;
   double cf1, cf2, cf3, p_top;
   double cfn, cfn1;  // top-face extrapolation weights (rk_addtend_dry.py:282-288)
+  int cfn_from_dn;   // formed by the threads that use them, from dn and dnw
 };
+
+// The top face's extrapolation weights: the caller's, or -- so that no caller has
+// to read dn and dnw back from the device for every step -- formed here.
+__device__ __forceinline__ void top_weights(const Grid &g, double &cfn, double &cfn1) {
+  cfn = g.cfn;
+  cfn1 = g.cfn1;
+  if (g.cfn_from_dn) {
+    const double dn = __ldg(g.dn + g.nz - 1), dnw = __ldg(g.dnw + g.nz - 1);
+    const double safe = fabs(dn) > 1.0e-30 ? dn : 1.0;
+    cfn = (0.5 * dnw + dn) / safe;
+    cfn1 = -0.5 * dnw / safe;
+  }
+}
 
 // The physics merge's w leaves (rk_addtend_dry; NULL = zero) for the w-face kernel.
 struct PhysW {

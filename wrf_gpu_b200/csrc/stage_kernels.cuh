@@ -184,7 +184,11 @@ __device__ __forceinline__ double dpn_large(const Grid &g, int m, int top_lid, P
   const int nz = g.nz;
   if (m == 0) return 0.5 * (g.cf1 * ps(0) + g.cf2 * ps(1) + g.cf3 * ps(2));
   if (m < nz) return 0.5 * (ld(g.fnm, m) * ps(m) + ld(g.fnp, m) * ps(m - 1));
-  if (top_lid) return 0.5 * (g.cfn * ps(nz - 1) + g.cfn1 * ps(nz - 2));
+  if (top_lid) {
+    double cfn, cfn1;
+    top_weights(g, cfn, cfn1);
+    return 0.5 * (cfn * ps(nz - 1) + cfn1 * ps(nz - 2));
+  }
   return 0.0;
 }
 

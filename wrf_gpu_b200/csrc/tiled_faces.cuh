@@ -678,12 +678,14 @@ __global__ void __launch_bounds__(TSX *TSY, WG_WFACE_MINB) k_wface_tiled(Grid g,
         // open-top face row: winds extrapolated with cfn/cfn1, weight 0.5
         // (core/rhs_ph.py:290-343)
         const double c1t = ld(g.c1f, nz), c2t = ld(g.c2f, nz);
+        double cfn, cfn1;
+        top_weights(g, cfn, cfn1);
         auto FY = [&](int jv) {
-          const double vt = g.cfn * ld(s.v, ix3(nz - 1, jv, i, ny + 1, nx)) + g.cfn1 * ld(s.v, ix3(nz - 2, jv, i, ny + 1, nx));
+          const double vt = cfn * ld(s.v, ix3(nz - 1, jv, i, ny + 1, nx)) + cfn1 * ld(s.v, ix3(nz - 2, jv, i, ny + 1, nx));
           return (c1t * ld(muv, ix2(jv, i, nx)) + c2t) * vt * ld(g.msfvy, ix2(jv, i, nx));
         };
         auto FX = [&](int iu) {
-          const double ut = g.cfn * ld(s.u, ix3(nz - 1, j, iu, ny, nx + 1)) + g.cfn1 * ld(s.u, ix3(nz - 2, j, iu, ny, nx + 1));
+          const double ut = cfn * ld(s.u, ix3(nz - 1, j, iu, ny, nx + 1)) + cfn1 * ld(s.u, ix3(nz - 2, j, iu, ny, nx + 1));
           return (c1t * ld(muu, ix2(j, iu, nx + 1)) + c2t) * ut * ld(g.msfux, ix2(j, iu, nx + 1));
         };
         auto PTo = [&](int dr, int dc) { return PT(ty + dr, tx + dc); };

@@ -347,7 +347,9 @@ def step_params(nl: OperationalNamelist) -> _capi.StepParams:
     p.const_nu_m2_s = float(nl.const_nu_m2_s)
     m = nl.metrics
     p.cf1, p.cf2, p.cf3, p.p_top = m.cf1, m.cf2, m.cf3, m.p_top
-    p.cfn, p.cfn1 = m.cfn()
+    # NaN: the kernels form the weights from dn and dnw (reading them back here
+    # would wait for the GPU on every call)
+    p.cfn, p.cfn1 = (math.nan, math.nan) if m.dn.numel() == m.dnw.numel() == nl.nz else m.cfn()
     return p
 
 
