@@ -1,0 +1,90 @@
+// Launch shape of the acoustic column kernels: host arithmetic alone (plain
+// C++, so that the rule can be checked without a GPU).
+#pragma once
+#include <cstddef>
+
+namespace wg {
+
+// Block shape.  Timed (us per launch, 433 x 433 x 50 / 256 x 256 x 50 /
+// 217 x 185 x 35 / 64 x 64 x 40): 16 columns x 26 lanes, 2 blocks per SM 619 /
+// 220 / 93 / 16.9; 16 x 17, 2 blocks 619 / 229 / 94 / 17.4; 16 x 17, 3 blocks
+// 630 / 223 / 99 / 19.5, 4 blocks 850 / 272 / 139 / 23.8 (56 registers spill);
+// 16 x 13, 3 blocks 684 / 251 / 97 / 22; 32 x 17, 1 block 630 / 243 / 120 /
+// 18.0; 32 x 26, 1 block 682 / 252 / 123 / 17.1; 32 x 32 761 / 276 / 137 / 18.8.
+#ifndef WG_COL_TY
+#define WG_COL_TY 26
+#endif
+constexpr int COL_TY = WG_COL_TY;
+constexpr int COL_NARR = 8;
+constexpr int COL_NMET = 9;    // level coefficients staged per block ...
+constexpr int COL_MET_NP = 4;  // ... for at most this many positions per lane
+// Column widths and level-lane counts the tuner tries (0: COL_TY).
+constexpr int COL_TX_CHOICES[] = {16, 32, 1};
+constexpr int COL_TY_CHOICES[] = {0, 13, 16};
+// The tallest column of the level-parallel kernel, at every width: what the
+// shared memory of a 32-column block holds.
+constexpr int COL_MAX_NZ = 112;
+// Width of the default column kernel: 1 selects the one-thread-per-column
+// streaming kernel (column_stream.cuh), 16 or 32 the level-parallel one
+// (column_tiled.cuh).
+#ifndef WG_COL_DEFAULT_WIDTH
+#define WG_COL_DEFAULT_WIDTH 16
+#endif
+constexpr int COL_DEFAULT_WIDTH = WG_COL_DEFAULT_WIDTH;
+static_assert(COL_DEFAULT_WIDTH == 1 || COL_DEFAULT_WIDTH == 16 || COL_DEFAULT_WIDTH == 32,
+              "the default column width is 1, 16 or 32");
+// Warps per block of the streaming kernel (each one row segment of 32
+// columns); two blocks per SM.
+#ifndef WG_CS_WARPS
+#define WG_CS_WARPS 4
+#endif
+constexpr int CS_WARPS = WG_CS_WARPS;
+
+inline size_t column_stream_smem_bytes(int nz) { return (size_t)2 * (nz + 1) * 32 * CS_WARPS * sizeof(double); }
+
+inline size_t column_tiled_smem_bytes(int nz, int tx, int np) {
+  return (size_t)(COL_NARR * tx + (np <= COL_MET_NP ? COL_NMET : 0)) * (nz + 1) * sizeof(double);
+}
+
+// Level lanes of a block and the positions per lane (np): the requested lanes,
+// or the fewest positions that COL_TY lanes reach (their number then trimmed so
+// that all lanes end together); at most 7 positions, or 14 for columns too tall
+// for 7 (nz > 118, 16-column blocks only).
+inline int column_tiled_lanes(int nz, int tx, int lanes, int &np) {
+  const int L = nz + 1, r0 = 32 / tx + 1;
+  int ty = lanes > 0 ? lanes : COL_TY;
+  np = (L + ty - 1) / ty;
+  if (np > 7) np = (L + COL_TY - 1) / COL_TY;
+  if (np > 7) np = 14;
+  if (np < 2) np = 2;
+  ty = (L + np - 1) / np;
+  return ty < r0 ? r0 : ty;
+}
+
+// The kernel and block for a requested column width (0: the default) and
+// level-lane count (0: the default; the streaming kernel has none).
+struct ColumnShape {
+  bool stream;       // one thread per column
+  int tx, ty, np;    // block (tx columns x ty lanes), positions per lane
+  size_t smem;       // dynamic shared memory, bytes
+  bool too_tall;     // more levels than the level-parallel kernel takes
+};
+
+inline ColumnShape column_shape(int nz, int width, int lanes) {
+  ColumnShape s{};
+  const int w = width > 0 ? width : COL_DEFAULT_WIDTH;
+  s.stream = w == 1;
+  if (s.stream) {
+    s.tx = 32;
+    s.ty = CS_WARPS;
+    s.smem = column_stream_smem_bytes(nz);
+    return s;
+  }
+  s.tx = w;
+  s.too_tall = nz > COL_MAX_NZ;
+  s.ty = column_tiled_lanes(nz, w, lanes, s.np);
+  s.smem = column_tiled_smem_bytes(nz, w, s.np);
+  return s;
+}
+
+}  // namespace wg

@@ -26,16 +26,9 @@
 #pragma once
 #include "dycore_common.cuh"
 #include "acoustic_kernels.cuh"
+#include "column_shape.cuh"
 
 namespace wg {
-
-// Warps per block (each one row segment of 32 columns); two blocks per SM.
-#ifndef WG_CS_WARPS
-#define WG_CS_WARPS 4
-#endif
-constexpr int CS_WARPS = WG_CS_WARPS;
-
-inline size_t column_stream_smem_bytes(int nz) { return (size_t)2 * (nz + 1) * 32 * CS_WARPS * sizeof(double); }
 
 // Coherent load of an array this kernel also writes.
 __device__ __forceinline__ double ldw(const double *p, size_t i) { return p[i]; }

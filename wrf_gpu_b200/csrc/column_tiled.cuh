@@ -27,18 +27,10 @@
 #pragma once
 #include "dycore_common.cuh"
 #include "acoustic_kernels.cuh"
+#include "column_shape.cuh"
 
 namespace wg {
 
-// Block shape.  Timed (us per launch, 433 x 433 x 50 / 256 x 256 x 50 /
-// 217 x 185 x 35 / 64 x 64 x 40): 16 columns x 26 lanes, 2 blocks per SM 619 /
-// 220 / 93 / 16.9; 16 x 17, 2 blocks 619 / 229 / 94 / 17.4; 16 x 17, 3 blocks
-// 630 / 223 / 99 / 19.5, 4 blocks 850 / 272 / 139 / 23.8 (56 registers spill);
-// 16 x 13, 3 blocks 684 / 251 / 97 / 22; 32 x 17, 1 block 630 / 243 / 120 /
-// 18.0; 32 x 26, 1 block 682 / 252 / 123 / 17.1; 32 x 32 761 / 276 / 137 / 18.8.
-#ifndef WG_COL_TY
-#define WG_COL_TY 26
-#endif
 // Resident blocks per SM requested from the register allocator, by width.
 #ifndef WG_COL_MINB16
 #define WG_COL_MINB16 2
@@ -50,22 +42,6 @@ namespace wg {
 #ifndef WG_COL_PREFETCH
 #define WG_COL_PREFETCH 1
 #endif
-constexpr int COL_TY = WG_COL_TY;
-constexpr int COL_NARR = 8;
-constexpr int COL_NMET = 9;    // level coefficients staged per block ...
-constexpr int COL_MET_NP = 4;  // ... for at most this many positions per lane
-// Column widths and level-lane counts the tuner tries (0: COL_TY).
-constexpr int COL_TX_CHOICES[] = {16, 32, 1};
-constexpr int COL_TY_CHOICES[] = {0, 13, 16};
-// The tallest column of a 32-wide block's shared memory.  The default is 16
-// wide but keeps this bound: it is the callers' limit unless they ask for 16.
-constexpr int COL_MAX_NZ = 112;
-// Width of the default column kernel: 1 selects the one-thread-per-column
-// streaming kernel (column_stream.cuh), 16 or 32 this level-parallel one.
-#ifndef WG_COL_DEFAULT_WIDTH
-#define WG_COL_DEFAULT_WIDTH 16
-#endif
-constexpr int COL_DEFAULT_WIDTH = WG_COL_DEFAULT_WIDTH;
 constexpr int col_minb(int tx) { return tx == 16 ? WG_COL_MINB16 : WG_COL_MINB; }
 // Levels per software-pipelined batch of the serial recurrences: the batch's
 // shared-memory operands are loaded before its first store, so the loads
@@ -106,25 +82,6 @@ __device__ __forceinline__ void column_prefetch(const Grid &g, const Acoustic &A
     pf(A.gamma);
     if (c.damp_opt == 3) pf(A.w_save);
   }
-}
-
-inline size_t column_tiled_smem_bytes(int nz, int tx, int np) {
-  return (size_t)(COL_NARR * tx + (np <= COL_MET_NP ? COL_NMET : 0)) * (nz + 1) * sizeof(double);
-}
-
-// Level lanes of a block and the positions per lane (np): the requested lanes,
-// or the fewest positions that COL_TY lanes reach (their number then trimmed so
-// that all lanes end together); at most 7 positions, or 14 for columns too tall
-// for 7 (nz > 118, 16-column blocks only).
-inline int column_tiled_lanes(int nz, int tx, int lanes, int &np) {
-  const int L = nz + 1, r0 = 32 / tx + 1;
-  int ty = lanes > 0 ? lanes : COL_TY;
-  np = (L + ty - 1) / ty;
-  if (np > 7) np = (L + COL_TY - 1) / COL_TY;
-  if (np > 7) np = 14;
-  if (np < 2) np = 2;
-  ty = (L + np - 1) / np;
-  return ty < r0 ? r0 : ty;
 }
 
 // PIN: compile in the boundary cadence's ring-0 pins of mu / muts / muave and

@@ -513,9 +513,8 @@ int wrfgpu_step_launch_count(const wrfgpu_step_params *p, int *launches) {
 
 namespace {
 
-// The column kernel and its launch shape for a column width (params; 0: the
-// default, 1: one thread per column, 16 / 32: level lanes) and a level-lane
-// count (0: the default).
+// The column kernel and its launch for a column width and level-lane count
+// (params; column_shape).
 struct ColumnLaunch {
   void (*kernel)(Grid, Acoustic, ColArgs, const double *, const double *);
   dim3 grid, block;
@@ -537,23 +536,19 @@ void (*column_tiled_kernel(int np))(Grid, Acoustic, ColArgs, const double *, con
 }
 
 ColumnLaunch column_launch(int nx, int ny, int nz, int width, int lanes, bool pins) {
+  const ColumnShape sh = column_shape(nz, width, lanes);
   ColumnLaunch c{};
-  if (width == 1) {
+  if (sh.stream) {
     c.kernel = pins ? k_column_stream<true> : k_column_stream<false>;
-    c.grid = dim3((nx + 31) / 32, (ny + CS_WARPS - 1) / CS_WARPS, 1);
-    c.block = dim3(32, CS_WARPS, 1);
-    c.smem = column_stream_smem_bytes(nz);
-    return c;
+    c.grid = dim3((nx + sh.tx - 1) / sh.tx, (ny + sh.ty - 1) / sh.ty, 1);
+  } else {
+    c.kernel = sh.tx == 16 ? (pins ? column_tiled_kernel<16, true>(sh.np) : column_tiled_kernel<16, false>(sh.np))
+                           : (pins ? column_tiled_kernel<32, true>(sh.np) : column_tiled_kernel<32, false>(sh.np));
+    c.grid = dim3((nx + sh.tx - 1) / sh.tx, ny, 1);
   }
-  const int tx = width > 0 ? width : COL_DEFAULT_WIDTH;
-  c.too_tall = width != 16 && nz > COL_MAX_NZ;
-  int np = 0;
-  const int ty = column_tiled_lanes(nz, tx, lanes, np);
-  c.kernel = tx == 16 ? (pins ? column_tiled_kernel<16, true>(np) : column_tiled_kernel<16, false>(np))
-                      : (pins ? column_tiled_kernel<32, true>(np) : column_tiled_kernel<32, false>(np));
-  c.grid = dim3((nx + tx - 1) / tx, ny, 1);
-  c.block = dim3(tx, ty, 1);
-  c.smem = column_tiled_smem_bytes(nz, tx, np);
+  c.block = dim3(sh.tx, sh.ty, 1);
+  c.smem = sh.smem;
+  c.too_tall = sh.too_tall;
   return c;
 }
 
@@ -1476,7 +1471,8 @@ int ac_forward(const wrfgpu_step_params &p, const Grid &g, const wrfgpu_acoustic
   if (int rc = check_launch("k_advance_uv")) return rc;
   k_div_h<<<grd(nx, ny, nz), blk2(), 0, stream>>>(g, A, specified, L.dvdxi, L.hdiv);
   if (int rc = check_launch("k_div_h")) return rc;
-  const ColumnLaunch col = column_launch(nx, ny, nz, 0, 0, false);
+  // (level-parallel: the streaming kernel works in place only)
+  const ColumnLaunch col = column_launch(nx, ny, nz, COL_DEFAULT_WIDTH == 1 ? 16 : COL_DEFAULT_WIDTH, 0, false);
   if (int rc = column_reserve(col)) return rc;
   col.kernel<<<col.grid, col.block, col.smem, stream>>>(g, A, ca, L.dvdxi, L.hdiv);
   return check_launch("k_column");
