@@ -401,9 +401,11 @@ int wrfgpu_acoustic_substep(const wrfgpu_step_params *params, const wrfgpu_metri
                             const wrfgpu_acoustic_consts *consts, wrfgpu_acoustic_work *x, double dts,
                             void *workspace, size_t workspace_bytes, cudaStream_t stream);
 
-/* x_out <- one acoustic substep of x, which is left as it is (no array of
- * x_out may be one of x); otherwise as wrfgpu_acoustic_substep.  For callers
- * that keep the substep's input, who otherwise copy it first. */
+/* x_out <- one acoustic substep of x, which is left as it is; otherwise as
+ * wrfgpu_acoustic_substep.  For callers that keep the substep's input, who
+ * otherwise copy it first.  No array of x_out may overlap an array of x, in
+ * its own place or another, or another array of x_out: refused with
+ * WRFGPU_ERR_BAD_SHAPE. */
 int wrfgpu_acoustic_substep_into(const wrfgpu_step_params *params, const wrfgpu_metrics *metrics,
                                  const wrfgpu_acoustic_consts *consts, const wrfgpu_acoustic_work *x,
                                  wrfgpu_acoustic_work *x_out, double dts, void *workspace, size_t workspace_bytes,

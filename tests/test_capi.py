@@ -206,6 +206,48 @@ def test_acoustic_substep_rejects_before_any_launch(lib):
     assert lib.wrfgpu_acoustic_workspace_size(ctypes.byref(_params(lib)), ctypes.byref(n)) == 0 and n.value > 0
 
 
+def test_acoustic_substep_into_refuses_shared_arrays(lib):
+    """x_out must not share memory with x -- in the same place, in another, or
+    in part -- nor any two of its arrays with each other; refused before any
+    launch (the pointers here are never read)."""
+    p = _params(lib)
+    nx, ny, nz = p.nx, p.ny, p.nz
+    size = dict(u=nz * ny * (nx + 1), v=nz * (ny + 1) * nx, w=(nz + 1) * ny * nx, ph=(nz + 1) * ny * nx,
+                ww=(nz + 1) * ny * nx, mu=ny * nx, muts=ny * nx, muave=ny * nx, mudf=ny * nx)
+    names = _capi.ACOUSTIC_WORK_FIELDS
+    bytes_of = {n: 8 * size.get(n, nz * ny * nx) for n in names}
+    m, c = _capi.Metrics(), _capi.AcousticConsts()
+    for n in _capi.ACOUSTIC_CONST_FIELDS:
+        setattr(c, n, 1 << 20)
+
+    def work(base):
+        out, at = {}, base
+        for n in names:  # back to back: neighbours touch and do not overlap
+            out[n] = at
+            at += bytes_of[n]
+        return out
+
+    x, o = work(1 << 24), work(1 << 28)
+    n = ctypes.c_size_t(0)
+    assert lib.wrfgpu_acoustic_workspace_size(ctypes.byref(p), ctypes.byref(n)) == 0
+
+    def refused(**change):
+        xs, os_ = _capi.AcousticWork(*[x[f] for f in names]), _capi.AcousticWork(*[{**o, **change}[f] for f in names])
+        return lib.wrfgpu_acoustic_substep_into(ctypes.byref(p), ctypes.byref(m), ctypes.byref(c), ctypes.byref(xs),
+                                                ctypes.byref(os_), 1.0, 1 << 32, n.value,
+                                                None) == _capi.WRFGPU_ERR_BAD_SHAPE
+
+    for f in names:
+        assert refused(**{f: x[f]}), f
+    assert refused(p=x["pm1"]) and refused(pm1=x["p"])  # swapped places
+    assert refused(p=x["pm1"], pm1=x["p"])
+    assert refused(w=x["u"] + bytes_of["u"] - 8) and refused(mu=x["theta_w"] + 8)  # parts
+    assert refused(muts=o["mu"]) and refused(ph=o["w"] + 8)  # two outputs in one place
+    xs = _capi.AcousticWork(*[x[f] for f in names])
+    assert lib.wrfgpu_acoustic_substep_into(ctypes.byref(p), ctypes.byref(m), ctypes.byref(c), ctypes.byref(xs),
+                                            ctypes.byref(xs), 1.0, 1 << 32, n.value, None) == _capi.WRFGPU_ERR_BAD_SHAPE
+
+
 def test_lateral_boundary_pass_rejects_before_any_launch(lib):
     ins, outs, lv = _capi.StepInputs(), _capi.StepOutputs(), _capi.LbcLeaves()
     assert lib.wrfgpu_apply_lateral_boundaries(ctypes.byref(_params(lib)), ctypes.byref(ins), ctypes.byref(lv),

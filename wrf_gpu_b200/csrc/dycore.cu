@@ -1394,6 +1394,12 @@ void ac_carve(const wrfgpu_step_params &p, Carver &cv, AcLayout &L) {
   }
 }
 
+// Whether n doubles at a and m doubles at b share memory.
+bool ranges_overlap(const double *a, size_t n, const double *b, size_t m) {
+  const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+  return p < q + m * sizeof(double) && q < p + n * sizeof(double);
+}
+
 double *const *work_ptrs(const wrfgpu_acoustic_work &x, double *out[14]) {
   double *v[14] = {x.u, x.v, x.w, x.ph, x.theta_w, x.t_2ave, x.p, x.pm1, x.al, x.ww, x.mu, x.muts, x.muave, x.mudf};
   for (int q = 0; q < 14; ++q) out[q] = v[q];
@@ -1508,9 +1514,15 @@ int ac_substep(const wrfgpu_step_params *p, const wrfgpu_metrics *m, const wrfgp
   double *w[14], *o[14];
   work_ptrs(*x, w);
   work_ptrs(*x_out, o);
-  for (int q = 0; q < 14; ++q) {
+  for (int q = 0; q < 14; ++q)
     if (w[q] == nullptr || o[q] == nullptr) return fail(WRFGPU_ERR_NULL_POINTER, "a work state pointer is NULL");
-    if (x != x_out && w[q] == o[q]) return fail(WRFGPU_ERR_BAD_SHAPE, "x_out must not alias x");
+  if (x != x_out) {  // every output against every input and the other outputs
+    size_t n[14];
+    ac_counts(dims_of(*p), n);
+    for (int q = 0; q < 14; ++q)
+      for (int r = 0; r < 14; ++r)
+        if (ranges_overlap(o[q], n[q], w[r], n[r]) || (r != q && ranges_overlap(o[q], n[q], o[r], n[r])))
+          return fail(WRFGPU_ERR_BAD_SHAPE, "x_out must not alias x, nor its arrays one another");
   }
   Carver cv{reinterpret_cast<char *>(workspace), 0, workspace_bytes, false};
   AcLayout L;
