@@ -199,7 +199,11 @@ typedef struct wrfgpu_step_inputs {
   const double *phys_u_save, *phys_v_save, *phys_w_save, *phys_ph_save, *phys_t_save;
 } wrfgpu_step_inputs;
 
-/* Step outputs: the returned OperationalCarry (operational_mode.py:2234-2265). */
+/* Step outputs: the returned OperationalCarry (operational_mode.py:2234-2265).
+ * The carry arrays (from t_2ave on) may be NULL where they are not wanted.  The
+ * step forms mudf .. ph_tend and the saves where they are asked for; one that
+ * shares memory with an input or another output is copied there after the
+ * last stage instead, at the price of the copy (mudf may be the input's). */
 typedef struct wrfgpu_step_outputs {
   double *u, *v, *w, *theta;
   double *p_total, *p_perturbation, *ph_total, *ph_perturbation;

@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <cmath>
+#include <functional>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -560,13 +561,99 @@ int column_reserve(const ColumnLaunch &c) {
   return WRFGPU_OK;
 }
 
+// The carry outputs formed in step-internal arrays, in the order in which the
+// shared ones are copied out.
+enum CarryOut {
+  CARRY_MUDF, CARRY_MUAVE, CARRY_MUTS, CARRY_PH_TEND, CARRY_U_SAVE, CARRY_V_SAVE, CARRY_W_SAVE, CARRY_PH_SAVE,
+  CARRY_MU_SAVE, CARRY_WW_SAVE, CARRY_N
+};
+
+struct Span {
+  const double *p;
+  size_t n;
+};
+
+// Whether n doubles at a and m doubles at b share memory.
+bool ranges_overlap(const double *a, size_t n, const double *b, size_t m) {
+  const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
+  return p < q + m * sizeof(double) && q < p + n * sizeof(double);
+}
+
+void carry_spans(const wrfgpu_step_params &p, const wrfgpu_step_outputs &o, Span c[CARRY_N]) {
+  const Dims d = dims_of(p);
+  c[CARRY_MUDF] = {o.mudf, d.s2}; c[CARRY_MUAVE] = {o.muave, d.s2}; c[CARRY_MUTS] = {o.muts, d.s2};
+  c[CARRY_PH_TEND] = {o.ph_tend, d.w}; c[CARRY_U_SAVE] = {o.u_save, d.u}; c[CARRY_V_SAVE] = {o.v_save, d.v};
+  c[CARRY_W_SAVE] = {o.w_save, d.w}; c[CARRY_PH_SAVE] = {o.ph_save, d.w}; c[CARRY_MU_SAVE] = {o.mu_save, d.s2};
+  c[CARRY_WW_SAVE] = {o.ww_save, d.w};
+}
+
+// Where each carry output is formed: in the caller's array, or -- when that
+// array shares memory with another one of the call (a caller may hand one
+// buffer to several outputs it does not want, or save over an input it no
+// longer needs) -- in the workspace, copied out after the last stage.
+class CarryPlacement {
+ public:
+  CarryPlacement(const wrfgpu_step_params &p, const wrfgpu_step_inputs &in, const wrfgpu_step_outputs &o, bool late)
+      : late_(late) {
+    const Dims d = dims_of(p);
+    carry_spans(p, o, out_);
+    auto add = [&](const double *q, size_t n) {
+      if (q != nullptr) all_[n_++] = {q, n};
+    };
+    add(in.u, d.u); add(in.v, d.v); add(in.w, d.w); add(in.theta, d.m); add(in.p_total, d.m);
+    add(in.p_perturbation, d.m); add(in.ph_total, d.w); add(in.ph_perturbation, d.w); add(in.mu_total, d.s2);
+    add(in.mu_perturbation, d.s2);
+    for (int s = 0; s < 6; ++s) add(in.q[s], d.m);
+    if (in.mudf != o.mudf) add(in.mudf, d.s2);  // (mudf may be advanced in place)
+    add(in.base_u, d.u); add(in.base_v, d.v); add(in.base_w, d.w); add(in.base_theta, d.m); add(in.base_mu, d.s2);
+    const size_t rows = (size_t)in.bdy_ntime * 4 * in.bdy_width * in.bdy_side_len;
+    add(in.u_bdy, rows * p.nz); add(in.v_bdy, rows * p.nz); add(in.theta_bdy, rows * p.nz);
+    add(in.ph_bdy, rows * (p.nz + 1)); add(in.w_bdy, rows * (p.nz + 1)); add(in.mu_bdy, rows);
+    if (p.physics) {
+      add(in.ru_tendf, d.u); add(in.rv_tendf, d.v); add(in.rw_tendf, d.w); add(in.t_tendf, d.m);
+      add(in.mu_tendf, d.s2); add(in.h_diabatic, d.m); add(in.phys_u_save, d.u); add(in.phys_v_save, d.v);
+      add(in.phys_w_save, d.w); add(in.phys_t_save, d.m);
+    }
+    add(o.u, d.u); add(o.v, d.v); add(o.w, d.w); add(o.theta, d.m); add(o.p_total, d.m); add(o.p_perturbation, d.m);
+    add(o.ph_total, d.w); add(o.ph_perturbation, d.w); add(o.mu_total, d.s2); add(o.mu_perturbation, d.s2);
+    for (int s = 0; s < 6; ++s) add(o.q[s], d.m);
+    add(o.t_2ave, d.m); add(o.ww, d.w); add(o.t_save, d.m);
+    for (const Span &c : out_) add(c.p, c.n);
+  }
+  // Put the work array behind carry output c.
+  void operator()(CarryOut c, double *&work) {
+    const Span &s = out_[c];
+    if (s.p == nullptr) return;
+    int hits = 0;  // itself, and any other
+    for (int k = 0; k < n_; ++k) hits += ranges_overlap(s.p, s.n, all_[k].p, all_[k].n) ? 1 : 0;
+    if (late_ || hits > 1)
+      src_[c] = work;
+    else
+      work = const_cast<double *>(s.p);
+  }
+  int copy_late(cudaStream_t stream) const {
+    for (int c = 0; c < CARRY_N; ++c)
+      if (src_[c] != nullptr && cudaMemcpyAsync(const_cast<double *>(out_[c].p), src_[c], out_[c].n * sizeof(double),
+                                                cudaMemcpyDeviceToDevice, stream) != cudaSuccess)
+        return fail(WRFGPU_ERR_CUDA, "carry output copy failed");
+    return WRFGPU_OK;
+  }
+
+ private:
+  bool late_;
+  Span out_[CARRY_N], all_[80];
+  int n_ = 0;
+  const double *src_[CARRY_N] = {};
+};
+
 // The RK3 step.  The forecast lead is `lead_seconds` (host; NaN = no lead:
 // boundary forcing off), or with `lead_dev` set a device-resident lead read
 // by the kernels that interpolate boundary strips in time (`lead_seconds` is
-// then only a non-NaN flag).
+// then only a non-NaN flag).  With `carry_late`, no carry output is written
+// before the last stage has finished (the callers' arrays may be shared).
 int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const wrfgpu_step_inputs *in,
                   const wrfgpu_step_outputs *out, double lead_seconds, const double *lead_dev, void *workspace,
-                  size_t workspace_bytes, cudaStream_t stream) {
+                  size_t workspace_bytes, cudaStream_t stream, bool carry_late = false) {
   if (pp == nullptr || mm == nullptr || in == nullptr || out == nullptr)
     return fail(WRFGPU_ERR_NULL_POINTER, "params/metrics/inputs/outputs is NULL");
   int rc = wrfgpu_step_params_validate(pp);
@@ -648,16 +735,15 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
   // wants them: the stage-2 state's u, v, w, ph', mu' (the saves) and, from the
   // last stage on, muts, muave, ph_tend and the stage omega (below).  Copying
   // them at the end took ten copies, 0.9 GB and 0.35 ms at 433 x 433 x 50 and
-  // about 3 us each on small grids.
-  auto redirect = [](double *&work, double *wanted) {
-    if (wanted != nullptr) work = wanted;
-  };
-  redirect(w.st[1].u, out->u_save);
-  redirect(w.st[1].v, out->v_save);
-  redirect(w.st[1].w, out->w_save);
-  redirect(w.st[1].ph_pert, out->ph_save);
-  redirect(w.st[1].mu_pert, out->mu_save);
-  redirect(w.mudf, out->mudf);
+  // about 3 us each on small grids.  Only an array that shares memory with an
+  // input or another output is still copied there.
+  CarryPlacement place(p, *in, *out, carry_late);
+  place(CARRY_U_SAVE, w.st[1].u);
+  place(CARRY_V_SAVE, w.st[1].v);
+  place(CARRY_W_SAVE, w.st[1].w);
+  place(CARRY_PH_SAVE, w.st[1].ph_pert);
+  place(CARRY_MU_SAVE, w.st[1].mu_pert);
+  place(CARRY_MUDF, w.mudf);
   // mudf carried across stages (operational_mode.py:2046)
   if (in->mudf != nullptr) {
     if (in->mudf != w.mudf && cudaMemcpyAsync(w.mudf, in->mudf, d.s2 * sizeof(double), cudaMemcpyDeviceToDevice,
@@ -773,10 +859,10 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
     const double dts = dts_rk[stage];
     StateW o = (stage == 2) ? final_out : w.st[stage];
     if (stage == 2) {
-      redirect(w.muts, out->muts);
-      redirect(w.muave, out->muave);
-      redirect(w.ph_tend, out->ph_tend);
-      redirect(specified ? w.ww_spec : w.rom, out->ww_save);
+      place(CARRY_MUTS, w.muts);
+      place(CARRY_MUAVE, w.muave);
+      place(CARRY_PH_TEND, w.ph_tend);
+      place(CARRY_WW_SAVE, specified ? w.ww_spec : w.rom);
     }
     if (!moist && stage < 2) {
       for (int q = 0; q < 6; ++q) o.q[q] = nullptr;  // moisture passes through untouched
@@ -1106,6 +1192,7 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
     }
     s = next;
   }
+  if ((rc = place.copy_late(stream)) != WRFGPU_OK) return rc;
   g_last_error.clear();
   return WRFGPU_OK;
 }
@@ -1243,6 +1330,18 @@ extern "C" int wrfgpu_rk3_step_batched(int n, const wrfgpu_step_params *params, 
   }
   if (n == 1) return wrfgpu_rk3_step(&params[0], &metrics[0], &in[0], &out[0], lead_seconds[0], workspace[0],
                                      workspace_bytes[0], stream);
+  // members that share a carry output (a buffer for arrays nobody wants) write it last
+  std::vector<Span> carry;
+  for (int m = 0; m < n; ++m) {
+    Span c[CARRY_N];
+    carry_spans(params[m], out[m], c);
+    for (const Span &q : c)
+      if (q.p != nullptr) carry.push_back(q);
+  }
+  std::sort(carry.begin(), carry.end(), [](const Span &a, const Span &b) { return std::less<const double *>()(a.p, b.p); });
+  bool shared = false;
+  for (size_t k = 1; k < carry.size(); ++k)
+    shared = shared || ranges_overlap(carry[k - 1].p, carry[k - 1].n, carry[k].p, carry[k].n);
   StreamPool *pool = nullptr;
   int rc = pool_for_current_device(&pool);
   if (rc) return rc;
@@ -1266,8 +1365,8 @@ extern "C" int wrfgpu_rk3_step_batched(int n, const wrfgpu_step_params *params, 
     load[best] += cells(m);
   }
   for (int m = 0; m < n; ++m) {
-    rc = wrfgpu_rk3_step(&params[m], &metrics[m], &in[m], &out[m], lead_seconds[m], workspace[m], workspace_bytes[m],
-                         pool->s[stream_of[m]]);
+    rc = rk3_step_impl(&params[m], &metrics[m], &in[m], &out[m], lead_seconds[m], nullptr, workspace[m],
+                       workspace_bytes[m], pool->s[stream_of[m]], shared);
     if (rc && first_err == WRFGPU_OK) {
       first_err = rc;
       first_msg = "member " + std::to_string(m) + ": " + g_last_error;
@@ -1392,12 +1491,6 @@ void ac_carve(const wrfgpu_step_params &p, Carver &cv, AcLayout &L) {
     L.s.fu[n] = cv.take(d.u);
     L.s.fv[n] = cv.take(d.v);
   }
-}
-
-// Whether n doubles at a and m doubles at b share memory.
-bool ranges_overlap(const double *a, size_t n, const double *b, size_t m) {
-  const uintptr_t p = reinterpret_cast<uintptr_t>(a), q = reinterpret_cast<uintptr_t>(b);
-  return p < q + m * sizeof(double) && q < p + n * sizeof(double);
 }
 
 double *const *work_ptrs(const wrfgpu_acoustic_work &x, double *out[14]) {
