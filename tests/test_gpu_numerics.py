@@ -57,11 +57,12 @@ def test_div_rcp_matches_cuda_division_bitwise(cuda_ready):
 
 
 def test_div_batch_matches_cuda_division_bitwise(cuda_ready):
-    """``div_batch`` (Newton reciprocal and Markstein correction, one special
-    test per batch) against ``/`` bit for bit: ordinary operands up to the ends
-    of its range (2^-500..2^500), all-ones and power-of-two mantissas, and
-    batches with a zero, infinite, NaN or out-of-range operand, which take
-    ``/`` for all three quotients."""
+    """``div_batch`` (reciprocal iteration and Markstein correction, one special
+    test per batch) against ``/`` bit for bit on drawn operands: ordinary ones up
+    to the ends of its range (2^-500..2^500; numerators from 2^-400), all-ones and
+    power-of-two mantissas, and batches with a zero, infinite, NaN or
+    out-of-range operand, which take ``/`` for all three quotients.  (Operands
+    that can differ are drawn for it below.)"""
     build.build()
     f = ctypes.CDLL(str(build.SELFTEST_LIB)).wrfgpu_selftest_div_batch
     f.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_long, ctypes.c_void_p]
@@ -86,3 +87,77 @@ def test_div_batch_matches_cuda_division_bitwise(cuda_ready):
         same = (g.view(np.uint64) == w.view(np.uint64)) | ((g == 0.0) & (w == 0.0)) | (np.isnan(g) & np.isnan(w))
         # a zero divided by a zero inside the fast path's range does not occur: b = 0 is out of range
         assert same.all(), (x[~same][:3], y[~same][:3], g[~same][:3], w[~same][:3])
+
+
+def _div_batch(x, y):
+    """(div_batch, CUDA's ``/``) of the operands, in groups of three."""
+    build.build()
+    f = ctypes.CDLL(str(build.SELFTEST_LIB)).wrfgpu_selftest_div_batch
+    f.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_long, ctypes.c_void_p]
+    f.restype = ctypes.c_int
+    n = x.size // 3
+    da, db = torch.as_tensor(x[:3 * n], device="cuda"), torch.as_tensor(y[:3 * n], device="cuda")
+    q1, q2 = torch.empty_like(da), torch.empty_like(da)
+    assert f(da.data_ptr(), db.data_ptr(), q1.data_ptr(), q2.data_ptr(), n,
+             torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    return q1.cpu().numpy(), q2.cpu().numpy()
+
+
+@pytest.mark.parametrize("emin,emax", [(-1074, -1022), (-1022, -1000), (-1000, -900), (-900, -500)])
+def test_div_batch_tiny_numerators(cuda_ready, emin, emax):
+    """Numerators down to the subnormals, alone and beside ordinary ones and
+    zeros: from 2^-900 up ``/``'s bits; below, where the residual a - b q may be
+    no double, within 2 ulp (the uncorrected quotient's 1.5 or the residual's
+    rounding, and the last rounding)."""
+    rng = np.random.default_rng(31)
+    n = 3 << 18
+    if emin < -1022:
+        a = rng.integers(1, 1 << 52, size=n, dtype=np.uint64).view(np.float64)
+    else:
+        a = _random_doubles(rng, n, emin, emax)
+    b = _random_doubles(rng, n, -2, 2)
+    mixed = a.copy()
+    mixed[::3] = _random_doubles(rng, a[::3].size, -3, 3)
+    mixed[1::6] = np.resize([0.0, -0.0], a[1::6].size)
+    for x, y in ((a, b), (a, _random_doubles(rng, n, -100, 499)), (a, _random_doubles(rng, n, -499, -100)), (mixed, b)):
+        g, w = _div_batch(x, y)
+        assert np.all(np.abs(g - w) <= 2.0 * np.spacing(np.abs(w))), (emin, emax)
+        big = (np.abs(x) >= 2.0 ** -900) | (x == 0.0)
+        assert np.array_equal(g[big], w[big]), (emin, emax)
+
+
+@pytest.mark.parametrize("kind", ["random", "near_one", "near_two", "below_two"])
+def test_div_batch_next_to_a_midpoint(cuda_ready, kind):
+    """The hardest operands: for an odd 53-bit b the a with a 2^54 = b m + 1 or
+    b m - 1, m odd, whose quotient lies 2^-53 / b of an ulp from the midpoint of
+    two doubles, where the bound on ``div_batch``'s error (half an ulp and 2^-50 of
+    one) allows the other neighbour for b > 2 (1 - 2^-6) and for no other b."""
+    rng = np.random.default_rng(17)
+    n = 90000
+    b = {"random": rng.integers(1 << 51, 1 << 52, size=n) * 2 + 1, "near_one": (1 << 52) + 2 * np.arange(n) + 1,
+         "near_two": (1 << 53) - 2 * np.arange(n) - 1,
+         "below_two": (1 << 53) - 2 * (2.0 ** rng.uniform(1, 46, n)).astype(np.int64) - 1}[kind]
+    a = np.empty(n)
+    for i, x in enumerate(map(int, b)):
+        inv = pow(x, -1, 1 << 54)
+        m, one = (inv, -1) if inv >> 53 else ((1 << 54) - inv, 1)
+        assert (x * m + one) % (1 << 54) == 0
+        a[i] = float((x * m + one) >> 54)
+    y = b.astype(np.float64)
+    g, w = _div_batch(a, y)
+    other = g != w
+    assert not np.any(other & (y < 2.0 ** 53 * (1.0 - 2.0 ** -6)))
+    assert np.all(np.abs(g - w)[other] == np.spacing(np.minimum(g, w))[other])
+
+
+def test_reciprocal_seed_is_as_good_as_div_batch_needs(cuda_ready):
+    """|1 - b y0| < 2^-19.9 of rcp.approx.ftz.f64, over every high word: e^3 is then
+    less than 2^-6 of an ulp of 1/b."""
+    build.build()
+    f = ctypes.CDLL(str(build.SELFTEST_LIB)).wrfgpu_selftest_rcp_seed
+    f.argtypes, f.restype = [ctypes.c_void_p, ctypes.c_void_p], ctypes.c_int
+    e0 = torch.empty(1 << 20, dtype=torch.float64, device="cuda")
+    assert f(e0.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert float(e0.max()) < 2.0 ** -19.9

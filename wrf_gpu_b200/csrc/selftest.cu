@@ -27,6 +27,22 @@ __global__ void k_div_batch_check(const double *a, const double *b, double *q_ba
   }
 }
 
+// Largest |1 - b y0| of the reciprocal's seed y0 over the divisors whose high
+// word is 1.0's plus i (the instruction reads the high word only, so the ends of the low
+// word are the extremes).
+__global__ void k_rcp_seed(double *e0) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 1 << 20) return;
+  double worst = 0.0;
+  for (int lo : {0, -1}) {
+    const double b = __hiloint2double(0x3ff00000 + i, lo);
+    double y0;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(b));
+    worst = fmax(worst, fabs(__fma_rn(-b, y0, 1.0)));
+  }
+  e0[i] = worst;
+}
+
 }  // namespace
 
 // q_rcp[i] = div_rcp(a[i], b[i], rb[i]) and q_div[i] = a[i] / b[i] (CUDA's
@@ -47,5 +63,11 @@ extern "C" int wrfgpu_selftest_div_batch(const double *a, const double *b, doubl
   if (groups <= 0) return 0;
   const int threads = 256;
   k_div_batch_check<<<(unsigned)((groups + threads - 1) / threads), threads, 0, stream>>>(a, b, q_batch, q_div, groups);
+  return cudaGetLastError() == cudaSuccess ? 0 : 3;
+}
+
+// e0 (2^20 doubles) = the seed's error over every high word of [1, 2).
+extern "C" int wrfgpu_selftest_rcp_seed(double *e0, cudaStream_t stream) {
+  k_rcp_seed<<<(1 << 20) / 256, 256, 0, stream>>>(e0);
   return cudaGetLastError() == cudaSuccess ? 0 : 3;
 }
