@@ -85,10 +85,12 @@ typedef struct wrfgpu_step_params {
   double cfn, cfn1;
   /* Kernel tile shapes (no counterpart in the reference; results do not
    * depend on them): levels per block of the level-marching stencil kernels
-   * (5, 10 or 25), level lanes of the column kernel (8, 13, 16 or 17) and
-   * its columns per block (16 or 32, or 1: one thread per column); 0 selects
-   * the built-in defaults (10, 26 and 16).  wrfgpu_autotune picks them per
-   * grid. */
+   * (5, 10 or 25), the most level lanes of the column kernel (8, 13, 16 or
+   * 17: its threads per column, each with ceil((nz + 1) / lanes) levels,
+   * trimmed to what those levels need; where that is more than four levels
+   * the built-in count is used) and its columns per block (16 or 32, or 1:
+   * one thread per column, which has no lanes); 0 selects the built-in
+   * defaults (10, 26 and 16).  wrfgpu_autotune picks them per grid. */
   int march_levels;
   int column_lanes;
   int column_width;

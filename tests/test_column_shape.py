@@ -1,8 +1,9 @@
 """The acoustic column kernels' launch shape (``csrc/column_shape.cuh``, host
 arithmetic) for every height, width and lane count the params accept, compiled
 here with the default column width of the build and with each of the others:
-a width of 1 -- asked for or the default -- is the streaming kernel, and every
-level-parallel block covers its levels within the kernel's bounds."""
+a width of 1 -- asked for or the default -- is the streaming kernel, every
+level-parallel block covers its levels within the kernel's bounds, and no
+request gets more than four positions per lane, where the kernel is slow."""
 
 from __future__ import annotations
 
@@ -59,6 +60,11 @@ def test_every_accepted_shape(tmp_path, default):
             continue
         # warp 0 is left to the serial phases, the next one forms the surface w
         assert 32 // tx + 1 <= ty <= max_lanes, what
-        assert 2 <= np_ <= 7 and ty * np_ >= nz + 1, what
+        assert ty * np_ >= nz + 1, what
+        # positions: those of the lanes asked for up to four, else the built-in count's
+        default_np = max(2, -(-(nz + 1) // max_lanes))
+        asked = -(-(nz + 1) // lanes) if lanes else default_np
+        assert np_ == max(2, asked if asked <= 4 else default_np), what
+        assert 2 <= np_ <= (4 if nz < 4 * max_lanes else 5), what
         # eight level arrays, and the level coefficients where they are staged
         assert smem >= 8 * tx * (nz + 1) * 8 and smem + 4 * tx * 8 <= SMEM_PER_BLOCK, what

@@ -46,18 +46,21 @@ inline size_t column_tiled_smem_bytes(int nz, int tx, int np) {
   return (size_t)(COL_NARR * tx + (np <= COL_MET_NP ? COL_NMET : 0)) * (nz + 1) * sizeof(double);
 }
 
-// Level lanes of a block and the positions per lane (np): the requested lanes,
-// or the fewest positions that COL_TY lanes reach (their number then trimmed so
-// that all lanes end together); at most 7 positions, or 14 for columns too tall
-// for 7 (nz > 118, 16-column blocks only).
+// Level lanes of a block and the positions per lane (np): the positions that the
+// requested lanes, or COL_TY lanes, need -- at least 2 -- and then the fewest lanes that
+// hold the column with them, so that all lanes end together.  A request that
+// needs more than COL_MET_NP positions gets COL_TY lanes': beyond that the kernel
+// spills hundreds of bytes per thread (us per launch, 160 x 150: 8 lanes, 7
+// positions at nz = 50: 208, against 160 for the kernel with 8 whole lanes that
+// the request used to name and 85 with 26; 13 lanes, 7 positions at nz = 80: 373,
+// 311 and 156).  COL_TY lanes themselves reach 5 positions, above nz = 103.
+constexpr int COL_MAX_NP = (COL_MAX_NZ + 1 + COL_TY - 1) / COL_TY;
 inline int column_tiled_lanes(int nz, int tx, int lanes, int &np) {
   const int L = nz + 1, r0 = 32 / tx + 1;
-  int ty = lanes > 0 ? lanes : COL_TY;
-  np = (L + ty - 1) / ty;
-  if (np > 7) np = (L + COL_TY - 1) / COL_TY;
-  if (np > 7) np = 14;
+  np = lanes > 0 ? (L + lanes - 1) / lanes : COL_MAX_NP;
+  if (lanes <= 0 || np > COL_MET_NP) np = (L + COL_TY - 1) / COL_TY;
   if (np < 2) np = 2;
-  ty = (L + np - 1) / np;
+  const int ty = (L + np - 1) / np;
   return ty < r0 ? r0 : ty;
 }
 

@@ -525,14 +525,12 @@ struct ColumnLaunch {
 
 template <int TX, bool PIN>
 void (*column_tiled_kernel(int np))(Grid, Acoustic, ColArgs, const double *, const double *) {
+  static_assert(COL_MAX_NP <= 5, "a column kernel for every number of positions");
   switch (np) {
-    case 1: case 2: return k_column_tiled<TX, 2, PIN>;
+    case 2: return k_column_tiled<TX, 2, PIN>;
     case 3: return k_column_tiled<TX, 3, PIN>;
     case 4: return k_column_tiled<TX, 4, PIN>;
-    case 5: return k_column_tiled<TX, 5, PIN>;
-    case 6: return k_column_tiled<TX, 6, PIN>;
-    case 7: return k_column_tiled<TX, 7, PIN>;
-    default: return k_column_tiled<TX, 14, PIN>;
+    default: return k_column_tiled<TX, 5, PIN>;
   }
 }
 
