@@ -14,6 +14,7 @@ product (``wrfgpu_acoustic_substep[_vjp]``, ``adjoint.AcousticOp``).
 
 from __future__ import annotations
 
+import ctypes
 from types import SimpleNamespace
 
 import numpy as np
@@ -102,6 +103,24 @@ def test_substep_forward_matches_oracle(cuda_ready, kind, rk):
         assert err <= TOL, (n, err)
 
 
+@pytest.mark.parametrize("nz", [51, 52, 78, 103, 104, 112])
+@pytest.mark.parametrize("specified", [False, True])
+def test_substep_forward_of_tall_columns_matches_oracle(cuda_ready, nz, specified):
+    """Two to five levels per lane of the column kernel; from five on (nz = 104)
+    it reads the level coefficients from global memory."""
+    case = cases.real_like_moist(18, 9, nz, hmax=500.0, specified=specified)
+    nl, a, dts, s = _stage(case, 3)
+    x = {cn: getattr(a, on).copy() for cn, on in WORK.items()}
+    op = _op(case, a, s, dts)
+    got = _cuda_step(op, x)
+    want = _oracle_step(nl, a, dts, x)
+    for n in _capi.ACOUSTIC_WORK_FIELDS:
+        # TOL is one substep's at 12 levels; the serial column recurrences (the sum of
+        # dmdt, the ww prefix, the two Thomas sweeps) carry rounding over nz
+        err = P.rel_err(got[n], want[n])
+        assert err <= TOL * max(1.0, nz / 12.0), (n, err)
+
+
 @pytest.mark.parametrize("kind", ["moist_periodic", "lid_damped", "moist_specified"])
 def test_substep_vjp_dot_product_against_finite_differences(cuda_ready, kind):
     case = _case(kind)
@@ -152,6 +171,35 @@ def test_substep_vjp_dot_product_against_finite_differences(cuda_ready, kind):
         dn = {m: (d[m] if m == n else np.zeros_like(d[m])) for m in d}
         lhs, rhs = _dot(cot, jd(oracle, dn)), float(np.sum(ci[n] * d[n]))
         assert abs(lhs - rhs) <= 1.0e-8 * (abs(lhs) + abs(rhs)) + floor, (n, lhs, rhs, floor)
+
+
+@pytest.mark.parametrize("kind", ["moist_periodic", "lid_damped", "moist_specified"])
+@pytest.mark.parametrize("rk", [1, 3])
+def test_substep_into_equals_the_substep_in_place(cuda_ready, kind, rk):
+    """Every element of the 14 outputs is written (NaN before the call), a
+    specified domain's frozen ring included, with the in-place call's bits; the
+    input stays as it is."""
+    case = _case(kind)
+    nl, a, dts, s = _stage(case, rk)
+    op = _op(case, a, s, dts)
+    rng = np.random.default_rng(8)
+    xs = []
+    for n in _capi.ACOUSTIC_WORK_FIELDS:  # every input non-zero, so that a ring value taken from elsewhere shows
+        f = getattr(a, WORK[n])
+        xs.append(torch.as_tensor(f + 1.0e-3 * rng.standard_normal(f.shape) * (1.0 + float(np.std(f))), device="cuda"))
+    keep = [t.clone() for t in xs]
+    want = [t.clone() for t in xs]
+    op.forward_(want)
+    outs = [torch.full_like(t, float("nan")) for t in xs]
+    x, o = op._work(xs), op._work(outs)
+    _capi.check(op.lib.wrfgpu_acoustic_substep_into(
+        ctypes.byref(op.params), ctypes.byref(op.metrics), ctypes.byref(op.consts), ctypes.byref(x), ctypes.byref(o),
+        op.dts, ctypes.c_void_p(op.workspace.data_ptr()), op.workspace.numel(),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    torch.cuda.synchronize()
+    for n, got, ref, now, was in zip(_capi.ACOUSTIC_WORK_FIELDS, outs, want, xs, keep):
+        assert torch.equal(got, ref), n
+        assert torch.equal(now, was), n
 
 
 def test_autograd_function_chains_two_substeps(cuda_ready):
