@@ -25,6 +25,13 @@ int main() {
         const wg::ColumnShape s = wg::column_shape(nz, w, l);
         std::printf("%d %d %d %d %d %d %d %zu %d\\n", nz, w, l, s.stream, s.tx, s.ty, s.np, s.smem, s.too_tall);
       }
+  for (int nz = 4; nz <= 112; ++nz) {
+    wg::ColumnRequest c[wg::COL_MAX_CANDIDATES];
+    const int n = wg::column_candidates(nz, c);
+    std::printf("candidates %d", nz);
+    for (int k = 0; k < n; ++k) std::printf(" %d %d", c[k].width, c[k].lanes);
+    std::printf("\\n");
+  }
   std::printf("%d %d %d\\n", wg::COL_TY, wg::COL_MAX_NZ, wg::CS_WARPS);
 }
 """
@@ -39,14 +46,16 @@ def _shapes(tmp_path, default):
     src.write_text(PROGRAM)
     flags = [f"-DWG_COL_DEFAULT_WIDTH={default}"] if default else []
     subprocess.run([gxx, "-std=c++17", *flags, "-I", str(build.CSRC), "-o", str(exe), str(src)], check=True)
-    rows = [tuple(map(int, line.split())) for line in
-            subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.splitlines()]
-    return rows[:-1], rows[-1]
+    lines = subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.splitlines()
+    ints = lambda line: tuple(map(int, line.split()))
+    tuner = [ints(line[len("candidates"):]) for line in lines if line.startswith("candidates")]
+    rows = [ints(line) for line in lines if not line.startswith("candidates")]
+    return rows[:-1], rows[-1], {t[0]: list(zip(t[1::2], t[2::2])) for t in tuner}
 
 
 @pytest.mark.parametrize("default", [None, 1, 16, 32])
 def test_every_accepted_shape(tmp_path, default):
-    rows, (max_lanes, max_nz, stream_warps) = _shapes(tmp_path, default)
+    rows, (max_lanes, max_nz, stream_warps), _ = _shapes(tmp_path, default)
     for nz, width, lanes, stream, tx, ty, np_, smem, too_tall in rows:
         what = (default, nz, width, lanes)
         wanted = width or default or 16
@@ -68,3 +77,15 @@ def test_every_accepted_shape(tmp_path, default):
         assert 2 <= np_ <= (4 if nz < 4 * max_lanes else 5), what
         # eight level arrays, and the level coefficients where they are staged
         assert smem >= 8 * tx * (nz + 1) * 8 and smem + 4 * tx * 8 <= SMEM_PER_BLOCK, what
+
+
+def test_the_tuner_times_no_launch_twice(tmp_path):
+    rows, _, tuner = _shapes(tmp_path, None)
+    launch = {r[:3]: r[3:7] for r in rows}
+    for nz, cands in tuner.items():
+        launches = [launch[nz, w, lanes] for w, lanes in cands]
+        assert len(set(launches)) == len(launches), (nz, cands)
+        # nothing that 17 or 13 lanes would give is missed
+        assert set(launches) == {launch[nz, w, lanes] for w in (1, 16, 32) for lanes in (0, 17, 13)}, (nz, cands)
+    assert tuner[50] == [(16, 0), (16, 17), (16, 13), (32, 0), (32, 17), (32, 13), (1, 0)]
+    assert tuner[20] == [(16, 0), (32, 0), (1, 0)]

@@ -2,6 +2,7 @@
 // C++, so that the rule can be checked without a GPU).
 #pragma once
 #include <cstddef>
+#include <initializer_list>
 
 namespace wg {
 
@@ -18,9 +19,6 @@ constexpr int COL_TY = WG_COL_TY;
 constexpr int COL_NARR = 8;
 constexpr int COL_NMET = 9;    // level coefficients staged per block ...
 constexpr int COL_MET_NP = 4;  // ... for at most this many positions per lane
-// Column widths and level-lane counts the tuner tries (0: COL_TY).
-constexpr int COL_TX_CHOICES[] = {16, 32, 1};
-constexpr int COL_TY_CHOICES[] = {0, 13, 16};
 // The tallest column of the level-parallel kernel, at every width: what the
 // shared memory of a 32-column block holds.
 constexpr int COL_MAX_NZ = 112;
@@ -88,6 +86,29 @@ inline ColumnShape column_shape(int nz, int width, int lanes) {
   s.ty = column_tiled_lanes(nz, w, lanes, s.np);
   s.smem = column_tiled_smem_bytes(nz, w, s.np);
   return s;
+}
+
+// The column widths and lane counts the tuner tries at this height, each a
+// different launch (lane counts that come to the same positions are one): the
+// default first, then 32 columns and one thread per column.  Returns their number.
+struct ColumnRequest {
+  int width, lanes;
+};
+constexpr int COL_MAX_CANDIDATES = 7;
+
+inline int column_candidates(int nz, ColumnRequest out[COL_MAX_CANDIDATES]) {
+  int n = 0;
+  for (int width : {16, 32, 1})
+    for (int lanes : {0, 17, 13}) {
+      const ColumnShape s = column_shape(nz, width, lanes);
+      bool seen = false;
+      for (int k = 0; k < n; ++k) {
+        const ColumnShape t = column_shape(nz, out[k].width, out[k].lanes);
+        seen = seen || (s.stream == t.stream && s.tx == t.tx && s.ty == t.ty && s.np == t.np);
+      }
+      if (!seen) out[n++] = {width, lanes};
+    }
+  return n;
 }
 
 }  // namespace wg

@@ -1406,21 +1406,17 @@ extern "C" int wrfgpu_autotune(wrfgpu_step_params *pp, const wrfgpu_metrics *mm,
   };
   wrfgpu_step_params best = *pp;
   float best_ms = 1e30f;
-  // column block shapes first (march levels at the default), then march levels;
-  // width 1 is the one-thread-per-column kernel (its lane count is unused)
-  for (int cw : COL_TX_CHOICES) {
-    for (int l : COL_TY_CHOICES) {
-      if (rc) break;
-      if (cw == 1 && l != COL_TY_CHOICES[0]) continue;
-      wrfgpu_step_params p = *pp;
-      p.column_width = cw;
-      p.column_lanes = l;
-      p.march_levels = 0;
-      float ms = 0.f;
-      rc = time_steps(p, &ms);
-      if (rc) break;
-      if (ms < best_ms) { best_ms = ms; best = p; }
-    }
+  // column block shapes first (march levels at the default), then march levels
+  ColumnRequest cand[COL_MAX_CANDIDATES];
+  const int ncand = column_candidates(pp->nz, cand);
+  for (int k = 0; k < ncand && rc == WRFGPU_OK; ++k) {
+    wrfgpu_step_params p = *pp;
+    p.column_width = cand[k].width;
+    p.column_lanes = cand[k].lanes;
+    p.march_levels = 0;
+    float ms = 0.f;
+    rc = time_steps(p, &ms);
+    if (rc == WRFGPU_OK && ms < best_ms) { best_ms = ms; best = p; }
   }
   for (int kcand : MARCH_KC_CHOICES) {
     if (rc) break;
