@@ -74,6 +74,20 @@ def test_batched_equals_individual_steps(cuda_ready):
     del graph
 
 
+def test_many_members_equal_individual_steps(cuda_ready):
+    """advance_uv's levels per thread depend on how many members share the GPU:
+    nine members, whose chunks differ from a lone domain's, bit for bit."""
+    cs = [cases.real_like_moist(22 + 3 * k, 18, 20 + k, hmax=500.0, specified=k % 2 == 1, seed=k) for k in range(9)]
+    nls = [dycore.OperationalNamelist.from_case(c) for c in cs]
+    carries = [dycore.carry_from_case(c) for c in cs]
+    bs = dycore.BatchStepper(nls)
+    outs = bs.alloc_carries(carries)
+    bs.step_into(carries, outs, lead_seconds=0.0)
+    torch.cuda.synchronize()
+    for nl, c, got in zip(nls, carries, outs):
+        _same(got, dycore.rk_scan_step(c, nl, lead_seconds=0.0))
+
+
 def test_autotune_picks_valid_shapes_and_results_do_not_depend_on_them(cuda_ready):
     case = cases.real_like_moist(64, 48, 20, hmax=800.0, specified=True)
     nl = dycore.OperationalNamelist.from_case(case)

@@ -13,6 +13,7 @@
 // stage-constant arrays and of u/v (finished by the face kernels), so a
 // substep has no intra-kernel race.
 #pragma once
+#include <algorithm>
 #include "dycore_common.cuh"
 
 namespace wg {
@@ -118,16 +119,27 @@ __device__ __forceinline__ double relax_weight_v(int j, int i, int y_len, int x_
 // 5 326, 3 359, 25 294, 50 300); against 17 levels for every grid:
 // 40 x 32 x 50 27.7 -> 10.7, 64 x 64 x 40 28.0 -> 14.4, 217 x 185 x 35
 // 70 -> 52, 150 x 150 x 45 47 -> 43.5 (256 x 256 x 50 and up unchanged).
+// Members of a batch share the GPU: `beside` counts the blocks per chunk that
+// they launch together, and a last wave that is not full is filled by their
+// other kernels, so waves count as they are.  (A member that counted alone took
+// chunks of two levels and their extra work; ms per captured step, 40 x 32 x 50,
+// alone / together: 4 members 1.17 / 1.16, 8 2.24 / 2.15, 32 8.94 / 8.61; 64 x 64
+// x 40: 16 members 7.94 / 7.82; two members of any size the same.)
 constexpr int UV_KC_MAX = 17;
-inline int advance_uv_levels(int nx, int ny, int nz) {
+inline double advance_uv_tiles(int nx, int ny) { return (double)((nx + 1 + 31) / 32) * ((ny + 1 + 3) / 4); }
+inline int advance_uv_levels(int nx, int ny, int nz, double beside = 0.0) {
   const double resident = 148.0 * WG_UV_MINB;  // blocks the GPU holds at once
-  const double tiles = (double)((nx + 1 + 31) / 32) * ((ny + 1 + 3) / 4);
+  const double own = advance_uv_tiles(nx, ny);
   int best = UV_KC_MAX;
   double best_cost = 1.0e300;
   for (int n = (nz + UV_KC_MAX - 1) / UV_KC_MAX; n <= nz; ++n) {
-    const int kc = (nz + n - 1) / n;
-    const double waves = tiles * ((nz + kc - 1) / kc) / resident;
-    const double cost = (waves < 4.0 ? ceil(waves) : waves) * (kc + 1.1);
+    const int kc = (nz + n - 1) / n, chunks = (nz + kc - 1) / kc;
+    double waves = std::max(own, beside) * chunks / resident;
+    if (beside > own)
+      waves = std::max(waves, 1.0);
+    else if (waves < 4.0)
+      waves = ceil(waves);
+    const double cost = waves * (kc + 1.1);
     if (cost < best_cost) {
       best_cost = cost;
       best = kc;

@@ -648,10 +648,12 @@ class CarryPlacement {
 // boundary forcing off), or with `lead_dev` set a device-resident lead read
 // by the kernels that interpolate boundary strips in time (`lead_seconds` is
 // then only a non-NaN flag).  With `carry_late`, no carry output is written
-// before the last stage has finished (the callers' arrays may be shared).
+// before the last stage has finished (the callers' arrays may be shared);
+// `uv_beside` is advance_uv's blocks per chunk of the domains that run
+// together (0: this one runs alone).
 int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const wrfgpu_step_inputs *in,
                   const wrfgpu_step_outputs *out, double lead_seconds, const double *lead_dev, void *workspace,
-                  size_t workspace_bytes, cudaStream_t stream, bool carry_late = false) {
+                  size_t workspace_bytes, cudaStream_t stream, bool carry_late = false, double uv_beside = 0.0) {
   if (pp == nullptr || mm == nullptr || in == nullptr || out == nullptr)
     return fail(WRFGPU_ERR_NULL_POINTER, "params/metrics/inputs/outputs is NULL");
   int rc = wrfgpu_step_params_validate(pp);
@@ -710,7 +712,7 @@ int rk3_step_impl(const wrfgpu_step_params *pp, const wrfgpu_metrics *mm, const 
   const bool specified = p.run_boundary && !p.bc_ideal;
   const double dt = p.dt;
   const int ns = p.acoustic_substeps;
-  const int uv_kc = advance_uv_levels(p.nx, p.ny, p.nz);
+  const int uv_kc = advance_uv_levels(p.nx, p.ny, p.nz, uv_beside);
   const int kc = (p.march_levels == 5 || p.march_levels == 25) ? p.march_levels : MARCH_KC;
   const double dt_rk[3] = {dt / 3.0, 0.5 * dt, dt};
   const double dts_rk[3] = {dt / 3.0, dt / (double)ns, dt / (double)ns};
@@ -1362,9 +1364,12 @@ extern "C" int wrfgpu_rk3_step_batched(int n, const wrfgpu_step_params *params, 
     stream_of[m] = best;
     load[best] += cells(m);
   }
+  // half the members that run at a time: they are seldom all in the same kernel
+  double uv_beside = 0.0;
+  for (int m = 0; m < n; ++m) uv_beside += advance_uv_tiles(params[m].nx, params[m].ny) * 0.5 * used / n;
   for (int m = 0; m < n; ++m) {
     rc = rk3_step_impl(&params[m], &metrics[m], &in[m], &out[m], lead_seconds[m], nullptr, workspace[m],
-                       workspace_bytes[m], pool->s[stream_of[m]], shared);
+                       workspace_bytes[m], pool->s[stream_of[m]], shared, uv_beside);
     if (rc && first_err == WRFGPU_OK) {
       first_err = rc;
       first_msg = "member " + std::to_string(m) + ": " + g_last_error;
