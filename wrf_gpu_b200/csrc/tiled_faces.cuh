@@ -126,8 +126,8 @@ template <typename F, bool DEG>
 __global__ void __launch_bounds__(TSX *TSY, WG_UFACE_MINB) k_uface_tiled(Grid g, StateR s, StateR ref, const double *ru,
                                                            const double *rv, const double *rom, Diag d,
                                                            const double *muu, const double *muus,
-                                                           const double *base_u, const double *rw, int top_lid,
-                                                           int run_boundary, UFaceOut o) {
+                                                           const double *base_u, int top_lid, int run_boundary,
+                                                           UFaceOut o) {
   constexpr bool deg = DEG;  // the specified-boundary advection degradation
   using TQ = Tile<3, 3>;
   using TR = Tile<1, 0>;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(TSX *TSY, WG_UFACE_MINB) k_uface_tiled(Grid g,
       const double muv_c = 0.5 * (mu2(js, ic) + mu2(jn, ic));
       return div_msf(ld(s.v, ix3(k, jv, ic, ny + 1, nx)) * (c1 * muv_c + c2), g.msfvx, g.rmsfvx, ix2(jv, ic, nx));
     };
-    auto rwq = [&](int kf, int ic) { return ld(rw, ix3(kf, j, ic, ny, nx)); };
+    auto rwq = [&](int kf, int ic) { return ld(d.rw, ix3(kf, j, ic, ny, nx)); };
     const double f_u = 0.5 * (ld(g.f, ix2(j, l, nx)) + ld(g.f, ix2(j, r, nx)));
     const double e_u = 0.5 * (ld(g.e, ix2(j, l, nx)) + ld(g.e, ix2(j, r, nx)));
     const double cosa_u = 0.5 * (ld(g.cosa, ix2(j, l, nx)) + ld(g.cosa, ix2(j, r, nx)));
@@ -279,8 +279,8 @@ template <typename F, bool DEG>
 __global__ void __launch_bounds__(TSX *TSY, WG_VFACE_MINB) k_vface_tiled(Grid g, StateR s, StateR ref, const double *ru,
                                                            const double *rv, const double *rom, Diag d,
                                                            const double *muv, const double *muvs,
-                                                           const double *base_v, const double *rw, int top_lid,
-                                                           int run_boundary, VFaceOut o) {
+                                                           const double *base_v, int top_lid, int run_boundary,
+                                                           VFaceOut o) {
   constexpr bool deg = DEG;  // the specified-boundary advection degradation
   using TQ = Tile<3, 3>;
   using TR = Tile<1, 1>;
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(TSX *TSY, WG_VFACE_MINB) k_vface_tiled(Grid g,
       const double muu_c = 0.5 * (mu2(jc, il) + mu2(jc, ir));
       return div_msf(ld(s.u, ix3(k, jc, iu, ny, nx + 1)) * (c1 * muu_c + c2), g.msfuy, g.rmsfuy, ix2(jc, iu, nx + 1));
     };
-    auto rwq = [&](int kf, int jc) { return ld(rw, ix3(kf, jc, i, ny, nx)); };
+    auto rwq = [&](int kf, int jc) { return ld(d.rw, ix3(kf, jc, i, ny, nx)); };
     const double f_v = 0.5 * (ld(g.f, ix2(sj, i, nx)) + ld(g.f, ix2(nj, i, nx)));
     const double e_v = 0.5 * (ld(g.e, ix2(sj, i, nx)) + ld(g.e, ix2(nj, i, nx)));
     const double sina_v = 0.5 * (ld(g.sina, ix2(sj, i, nx)) + ld(g.sina, ix2(nj, i, nx)));
