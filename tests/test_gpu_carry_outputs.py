@@ -49,7 +49,8 @@ def _same(ref, got, carry=()):
 
 
 @pytest.mark.parametrize("kind", ["periodic", "specified", "cadence"])
-@pytest.mark.parametrize("left_out", [ORDER, ORDER[::2], ORDER[1::2], ("ww_save",), ("mudf",), ("u_save", "mu_save")])
+@pytest.mark.parametrize("left_out", [tuple(P.CARRY_KEYS), ORDER, ORDER[::2], ORDER[1::2], ("ww_save",), ("mudf",),
+                                      ("u_save", "mu_save"), ("t_2ave", "ww", "t_save")])
 def test_left_out(cuda_ready, kind, left_out):
     case = _case(kind)
     got = _step(case, lambda c, o: [setattr(o, f, None) for f in left_out])
