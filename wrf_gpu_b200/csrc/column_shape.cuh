@@ -12,6 +12,9 @@ namespace wg {
 // 630 / 223 / 99 / 19.5, 4 blocks 850 / 272 / 139 / 23.8 (56 registers spill);
 // 16 x 13, 3 blocks 684 / 251 / 97 / 22; 32 x 17, 1 block 630 / 243 / 120 /
 // 18.0; 32 x 26, 1 block 682 / 252 / 123 / 17.1; 32 x 32 761 / 276 / 137 / 18.8.
+// Above 51 levels the lanes hold three or four levels and spill (52 and 196
+// bytes per thread); against the 32 x 17 form still 422 -> 299 at 301 x 301 x 52,
+// 731 -> 373 at 60 levels, 909 -> 580 at 80, 1090 -> 813 at 95.
 #ifndef WG_COL_TY
 #define WG_COL_TY 26
 #endif

@@ -22,7 +22,7 @@
 // the surface w formed by its own warp at the start; one prefetch per line;
 // few positions (26 lanes) on 16 columns, two blocks per SM, so that one
 // block's serial phases overlap the other's loads.
-// 433 x 433 x 50: 0.776 -> 0.619 ms per launch (2.9 -> 3.6 TB/s of the 2.25 GB);
+// 433 x 433 x 50: 0.776 -> 0.615 ms per launch (2.25 GB at 2.9 TB/s -> 2.04 GB at 3.3);
 // 256 x 256 x 50: 0.286 -> 0.220 ms; 64 x 64 x 40: 29.5 -> 16.9 us.
 #pragma once
 #include "dycore_common.cuh"
